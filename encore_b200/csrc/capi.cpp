@@ -163,7 +163,10 @@ Launch resolve_launch(const enc_launch_opts* o, int kind, int width) {
   if (o) {
     if (o->block_threads > 0) L.block = o->block_threads;
     if (o->blocks_per_sm > 0) L.blocks_per_sm = o->blocks_per_sm;
-    if (o->chunk > 0) L.chunk = o->chunk;
+    if (o->chunk > 0) {
+      L.chunk = o->chunk;
+      L.fixed_chunk = true;
+    }
     if (o->stack_depth > 0) L.stack = o->stack_depth;
   }
   return L;

@@ -168,6 +168,7 @@ struct Launch {
   int block = 128;
   int blocks_per_sm = 4;
   int chunk = 32;
+  bool fixed_chunk = false;  // the caller chose `chunk`
   int stack = 32;
   // Closest hit with one triangle loop per lane instead of the warp-wide
   // triangle rounds: the host-buffer pipeline uses it (see host_form).
