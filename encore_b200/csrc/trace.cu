@@ -14,7 +14,8 @@
 //    with direction sign bits octm); widths 2 and 4 sort hit children by
 //    entry distance.  MULTI launches trace many scenes' batches at once.
 //  * kd_trace<CLAMP>: the reference's kd-tree walk (Kdtree.cpp:682-784), one
-//    thread per ray, over the flattened kd layout.  Bit-exact parity mode.
+//    lane per ray with the leaves' items tested by the whole warp, over the
+//    flattened kd layout.  Bit-exact parity mode.
 //
 // The triangle test follows TrianglePrim::intersect (TrianglePrim.cpp:204-248)
 // operation for operation: every product and sum is a separately rounded FP32
@@ -936,155 +937,301 @@ struct KdParams {
   const uint32_t* items;
   const float4* tris;  // triangle-ID order
   const float4* rays;
-  const uint32_t* order;  // null, or: the i-th ray walked is ray order[i] (binned batches)
+  const uint32_t* order;  // null, or: queue index q walks ray order[q] (binned batches)
   void* out;
   uint32_t* status;
+  unsigned* counter;
+  unsigned share;  // > 0: warp w walks queue indices [w * share, (w + 1) * share)
   unsigned nrays, nnodes, nitems, ntris;
   float lo[3], hi[3];  // root box min corner and pos + size
 };
 
-// Deferred far children of the walk: at most one per level, so a tree of
-// depth <= 32 (the reference's depth limit 11 + 1.3 ln N stays below 32 up
-// to about 10M triangles) needs 32 entries; deeper trees get 64.  The
-// stack lives in local memory: the smaller one halves its traffic.
-// Resident blocks per SM for the kd walk: one thread walks one ray, so its
-// latency is hidden only by other warps.  At 10 blocks (48 registers, a
-// 16-byte spill) it ran 6.8 % faster than at 8 (53 registers); 12 and 16
-// spill 80 and 216 bytes and lose.
-constexpr int kKdBlocks = 10;
+// The walk alternates between two phases, each with most of the warp's lanes
+// at work.  One thread per ray that tested its own leaves ran 5.8 lanes per
+// instruction: a lane at a leaf looped over its items while the others waited
+// (3.69 G warp instructions for 1M rays on a 524,288-triangle field).
+//   1. Every lane steps through inner nodes and empty leaves until it stands
+//      at a leaf with items; the phase ends once kKdLeave or fewer lanes are
+//      still walking (they go on next time).
+//   2. The items of all those leaves form one list that the warp tests 32 at
+//      a time, lane w testing item w with its owner's ray.  The reference tests
+//      a leaf's items in order and keeps t < best; the smallest (t, position in
+//      the list) below the owner's best is the same item.
+// Lanes whose walk is over take new rays once kKdRefill of them are idle, so
+// the set-up's six divisions run for several lanes at a time.
+// Measured on that batch: 5,190 us one thread per ray, 2,114 us now (1.60 G
+// warp instructions at 25 lanes); kKdLeave 4 / 8 / 12 / 20 / 24: 2,308 / 2,210 /
+// 2,152 / 2,155 / 2,260; kKdRefill 1 / 4 / 16: within 1 %; 6 / 7 / 9 / 10 blocks
+// per SM: 2,441 / 2,253 / 2,200 / 2,560.  What bounds it now: issue (73 %
+// active) and the latency of its dependent node, item and triangle loads (L2 hit
+// rate 99 %).
+constexpr int kKdBlocks = 8;
+constexpr int kKdLeave = 16;
+constexpr int kKdRefill = 8;
+constexpr unsigned kKdChunk = 32;  // rays a warp takes from the queue at a time
+// Deferred far children of the walk: at most one per level.  The first entries
+// live in shared memory, which most rays never leave; deeper ones in local
+// memory.
+constexpr int kKdShared = 12;
+constexpr int kKdStack = 64;
+// Items of one leaf listed at a time: bounds the list of 32 leaves.
+constexpr uint32_t kKdLeafItems = 1u << 16;
 
-template <bool CLAMP, bool ANY, int kKdStack>
+template <bool CLAMP, bool ANY>
 __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
-  for (unsigned qi = blockIdx.x * blockDim.x + threadIdx.x; qi < P.nrays;
-       qi += gridDim.x * blockDim.x) {
-    const unsigned ray = P.order ? __ldg(P.order + qi) : qi;
-    if (ray >= P.nrays) {  // an order entry outside the batch: skipped and reported
-      atomicOr(P.status, kStatusBounds);
-      continue;
-    }
-    const float4 r0 = __ldg(P.rays + 2 * (size_t)ray);
-    const float4 r1 = __ldg(P.rays + 2 * (size_t)ray + 1);
-    const float o[3] = {r0.x, r0.y, r0.z};
-    const float d[3] = {r1.x, r1.y, r1.z};
-    const float rtmin = r0.w, rtmax = r1.w;
-    const float inv[3] = {__fdiv_rn(1.f, d[0]), __fdiv_rn(1.f, d[1]), __fdiv_rn(1.f, d[2])};
-    float best_t = INFINITY, bu = 0.f, bv = 0.f;
-    int best_id = -1;
-    // m_Bounds.Intersect(r, tmin, tmax)  (AABB.cpp:117-143)
-    float t0 = 0.f, t1 = INFINITY;
-    bool in = true;
-    for (int i = 0; i < 3 && in; ++i) {
-      float tin = __fdiv_rn(fs(P.lo[i], o[i]), d[i]);
-      float tout = __fdiv_rn(fs(P.hi[i], o[i]), d[i]);
-      if (tin > tout) {
-        float tt = tin;
-        tin = tout;
-        tout = tt;
+  __shared__ uint2 s_stack[kKdShared][128];
+  __shared__ float s_o[3][128], s_d[3][128], s_inv[3][128];
+  __shared__ float2 s_lim[128];              // the ray's tmin and tmax
+  __shared__ unsigned long long s_key[128];  // best candidate of the lane's leaf
+  __shared__ float4 s_hit[128];              // t, u, v, ID of the ray's closest hit so far
+  __shared__ uint8_t s_own[128];             // r-th lane of the warp that has leaf items
+  uint2 deep[kKdStack - kKdShared];               // stack entries beyond the shared ones
+  const unsigned tid = threadIdx.x, lane = tid & 31u, wbase = tid & ~31u;
+  const unsigned lt = lanemask_lt();
+
+  unsigned pool_next = 0, pool_end = 0;
+  bool exhausted = false;
+  if (P.share) {
+    const unsigned w = blockIdx.x * (blockDim.x >> 5) + (tid >> 5);
+    pool_next = min(w * P.share, P.nrays);
+    pool_end = min(pool_next + P.share, P.nrays);
+  }
+
+  bool active = false;
+  unsigned ray = 0, steps = 0;
+  uint32_t node = 0;
+  uint32_t cnt = 0, beg = 0;  // pending leaf (cnt > 0): its items
+  int sp = 0;
+  float tmin = 0.f, tmax = 0.f, tend = 0.f, best_t = INFINITY;
+
+  while (true) {
+    // ---- refill idle lanes ------------------------------------------------
+    unsigned idle = __ballot_sync(kFull, !active);
+    if (idle && !exhausted && (idle == kFull || __popc(idle) >= kKdRefill)) {
+      bool fresh = false;
+      while (idle && !exhausted) {
+        if (pool_next >= pool_end) {
+          unsigned b = P.nrays;
+          if (!P.share) {
+            if (lane == 0) b = atomicAdd(P.counter, kKdChunk);
+            b = __shfl_sync(kFull, b, 0);
+          }
+          if (b >= P.nrays) {
+            exhausted = true;
+            break;
+          }
+          pool_next = b;
+          pool_end = min(b + kKdChunk, P.nrays);
+        }
+        const unsigned avail = pool_end - pool_next;
+        const unsigned rank = __popc(idle & lt);
+        if (((idle >> lane) & 1u) && rank < avail) {
+          ray = pool_next + rank;
+          active = fresh = true;
+          if (P.order) {
+            ray = __ldg(P.order + ray);
+            if (ray >= P.nrays) {  // an order entry outside the batch: skipped and reported
+              atomicOr(P.status, kStatusBounds);
+              active = fresh = false;
+            }
+          }
+        }
+        pool_next += min(avail, (unsigned)__popc(idle));
+        idle = __ballot_sync(kFull, !active);
       }
-      t0 = tin > t0 ? tin : t0;
-      t1 = tout < t1 ? tout : t1;
-      if (t0 > t1) in = false;
+      if (fresh) {
+        const float4 r0 = __ldg(P.rays + 2 * (size_t)ray);
+        const float4 r1 = __ldg(P.rays + 2 * (size_t)ray + 1);
+        const float o[3] = {r0.x, r0.y, r0.z};
+        const float d[3] = {r1.x, r1.y, r1.z};
+        // m_Bounds.Intersect(r, tmin, tmax)  (AABB.cpp:117-143)
+        float t0 = 0.f, t1 = INFINITY;
+        bool in = true;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          s_o[i][tid] = o[i];
+          s_d[i][tid] = d[i];
+          s_inv[i][tid] = __fdiv_rn(1.f, d[i]);
+          if (in) {
+            float tin = __fdiv_rn(fs(P.lo[i], o[i]), d[i]);
+            float tout = __fdiv_rn(fs(P.hi[i], o[i]), d[i]);
+            if (tin > tout) {
+              const float tt = tin;
+              tin = tout;
+              tout = tt;
+            }
+            t0 = tin > t0 ? tin : t0;
+            t1 = tout < t1 ? tout : t1;
+            if (t0 > t1) in = false;
+          }
+        }
+        s_lim[tid] = make_float2(r0.w, r1.w);
+        s_hit[tid] = make_float4(INFINITY, 0.f, 0.f, __int_as_float(-1));
+        best_t = INFINITY;
+        tmin = t0;
+        tmax = tend = t1;
+        sp = 0;
+        node = 0;
+        steps = 0;
+        cnt = 0;
+        if (!in) node = kNoItem;  // no walk: ends below as a miss
+      }
     }
-    if (in) {
-      float tmin = t0, tmax = t1;
-      uint32_t st_node[kKdStack];
-      float st_min[kKdStack], st_max[kKdStack];
-      int sp = 0;
-      uint32_t node = 0;
-      unsigned steps = 0;
-      while (true) {
-        if (++steps > kMaxSteps) {
-          atomicOr(P.status, kStatusWatchdog);
-          best_id = -1;
-          break;
-        }
-        if (best_t < tmin) break;
-        if (node >= P.nnodes) {
-          atomicOr(P.status, kStatusBounds);
-          best_id = -1;
-          break;
-        }
-        const KdNode n = P.nodes[node];
-        if ((n.word0 & 3u) != 3u) {
-          const int axis = (int)(n.word0 & 3u);
-          float split = __uint_as_float(n.word0);
+    if (__ballot_sync(kFull, active) == 0) break;
+
+    // The walk returns to the far child deferred last.  The interval it was
+    // deferred with ended where the one below it on the stack begins (or at
+    // the root box's exit): a push sets tmax to the new entry's tplane and a
+    // pop restores the value before it, so an entry needs no tmax of its own.
+    auto entry = [&](int i) { return i < kKdShared ? s_stack[i][tid] : deep[i - kKdShared]; };
+    auto pop = [&]() {
+      if (sp == 0) return false;
+      --sp;
+      const uint2 e = entry(sp);
+      node = e.x;
+      tmin = __uint_as_float(e.y);
+      tmax = sp > 0 ? __uint_as_float(entry(sp - 1).y) : tend;
+      return true;
+    };
+
+    // ---- walk until the lanes stand at leaves -----------------------------
+    bool fin = active && node == kNoItem;  // the ray's walk is over
+    bool lost = false;                     // stopped at a bound: reported as a miss
+    while (true) {
+      const bool walking = active && !fin && cnt == 0;
+      const unsigned wm = __ballot_sync(kFull, walking);
+      const unsigned at_leaf = __ballot_sync(kFull, cnt != 0);
+      if (wm == 0 || (at_leaf != 0 && __popc(wm) <= kKdLeave)) break;
+      if (!walking) continue;
+      if (++steps > kMaxSteps) {
+        atomicOr(P.status, kStatusWatchdog);
+        fin = lost = true;
+      } else if (best_t < tmin) {
+        fin = true;
+      } else if (node >= P.nnodes) {
+        atomicOr(P.status, kStatusBounds);
+        fin = lost = true;
+      } else {
+        const uint2 n = __ldg(reinterpret_cast<const uint2*>(P.nodes) + node);
+        const uint32_t axis = n.x & 3u;
+        if (axis != 3u) {
+          float split = __uint_as_float(n.x);
           split = (split > -0.001f && split < 0.001f) ? 0.0f : split;
-          // the axis's origin and reciprocal by select, not by indexing the
-          // arrays with the runtime axis (which would put them in local memory)
-          const float oa = axis == 0 ? o[0] : (axis == 1 ? o[1] : o[2]);
-          const float ia = axis == 0 ? inv[0] : (axis == 1 ? inv[1] : inv[2]);
+          const float oa = s_o[axis][tid], ia = s_inv[axis][tid];
           const float tplane = fm(fs(split, oa), ia);
           const bool below = oa <= split;
-          const uint32_t first = below ? n.word1 : n.word1 + 1;
-          const uint32_t second = below ? n.word1 + 1 : n.word1;
+          const uint32_t first = below ? n.y : n.y + 1;
+          const uint32_t second = below ? n.y + 1 : n.y;
           if (tplane == 0.0f) {
             node = ia > 0.0f ? second : first;
           } else if (tplane >= tmax || tplane < 0.0f) {
             node = first;
           } else if (tplane <= tmin) {
             node = second;
+          } else if (sp >= kKdStack) {
+            atomicOr(P.status, kStatusStack);
+            fin = lost = true;
           } else {
-            if (sp >= kKdStack) {
-              atomicOr(P.status, kStatusStack);
-              best_id = -1;
-              break;
-            }
-            st_node[sp] = second;
-            st_min[sp] = tplane;
-            st_max[sp] = tmax;
+            const uint2 e = make_uint2(second, __float_as_uint(tplane));
+            if (sp < kKdShared) s_stack[sp][tid] = e;
+            else deep[sp - kKdShared] = e;
             ++sp;
             node = first;
             tmax = tplane;
           }
         } else {
-          const uint32_t cnt = n.word0 >> 2;
-          const uint32_t beg = n.word1;
+          cnt = n.x >> 2;
+          beg = n.y;
           if ((size_t)beg + cnt > P.nitems) {
             atomicOr(P.status, kStatusBounds);
-            best_id = -1;
-            break;
-          }
-          for (uint32_t k = 0; k < cnt; ++k) {
-            const uint32_t id = __ldg(P.items + beg + k);
-            if (id >= P.ntris) {
-              atomicOr(P.status, kStatusBounds);
-              continue;
-            }
-            const float4* tp = P.tris + 3 * (size_t)id;
-            float t, u, v;
-            if (tri_test<CLAMP>(__ldg(tp), __ldg(tp + 1), __ldg(tp + 2), o[0], o[1], o[2], d[0],
-                                d[1], d[2], rtmin, t, u, v) &&
-                t < best_t) {
-              best_t = t;
-              best_id = (int)id;
-              bu = u;
-              bv = v;
-            }
-          }
-          if (sp > 0) {
-            --sp;
-            node = st_node[sp];
-            tmin = st_min[sp];
-            tmax = st_max[sp];
-          } else {
-            break;
+            cnt = 0;
+            fin = lost = true;
+          } else if (cnt == 0 && !pop()) {  // an empty leaf
+            fin = true;
           }
         }
       }
     }
-    // IsInShadow form: closest hit && t < distance; closest: hits at or
-    // beyond the ray's tmax are reported as misses.
-    const bool hit = best_id >= 0 && best_t < rtmax;
-    if (ANY) {
-      reinterpret_cast<uint8_t*>(P.out)[ray] = hit ? 1 : 0;
-    } else {
-      int4 h;
-      h.x = hit ? best_id : -1;
-      h.y = hit ? __float_as_int(best_t) : 0;
-      h.z = hit ? __float_as_int(bu) : 0;
-      h.w = hit ? __float_as_int(bv) : 0;
-      reinterpret_cast<int4*>(P.out)[ray] = h;
+
+    // ---- the warp tests the items of its lanes' leaves together -----------
+    const unsigned leaves = __ballot_sync(kFull, cnt != 0);
+    if (leaves) {
+      const uint32_t take = min(cnt, kKdLeafItems);
+      uint32_t excl = take;  // becomes the lane's first item in the warp's list
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, excl, d);
+        if ((int)lane >= d) excl += v;
+      }
+      const uint32_t total = __shfl_sync(kFull, excl, 31);
+      excl -= take;
+      if (take) s_own[wbase + __popc(leaves & lt)] = (uint8_t)lane;
+      s_key[tid] = ~0ull;
+      __syncwarp();
+      for (uint32_t base = 0; base < total; base += 32) {
+        // the owner of item base + lane: the last lane whose list starts at
+        // or before it
+        const bool starts = take && excl >= base && excl < base + 32;
+        const uint32_t first = __reduce_or_sync(kFull, starts ? 1u << (excl - base) : 0u);
+        const unsigned before = __popc(__ballot_sync(kFull, take && excl < base));
+        const unsigned own = s_own[wbase + before + __popc(first & (lt | (1u << lane))) - 1];
+        const uint32_t oexcl = __shfl_sync(kFull, excl, own);
+        const uint32_t obeg = __shfl_sync(kFull, beg, own);
+        const float obest = __shfl_sync(kFull, best_t, own);
+        const unsigned ot = wbase + own;
+        bool cand = false;
+        unsigned long long key = 0;
+        float t = 0.f, u = 0.f, v = 0.f;
+        uint32_t id = 0;
+        if (base + lane < total) {
+          const uint32_t k = base + lane - oexcl;
+          id = __ldg(P.items + obeg + k);
+          if (id >= P.ntris) {
+            atomicOr(P.status, kStatusBounds);
+          } else {
+            const float4* tp = P.tris + 3 * (size_t)id;
+            if (tri_test<CLAMP>(__ldg(tp), __ldg(tp + 1), __ldg(tp + 2), s_o[0][ot], s_o[1][ot],
+                                s_o[2][ot], s_d[0][ot], s_d[1][ot], s_d[2][ot], s_lim[ot].x, t, u,
+                                v) &&
+                t < obest) {
+              cand = true;
+              // -0 and +0 are one distance: the first of them in the list wins
+              key = ((unsigned long long)order_key(t == 0.0f ? 0.0f : t) << 32) | k;
+              atomicMin(&s_key[ot], key);
+            }
+          }
+        }
+        __syncwarp();
+        if (cand && s_key[ot] == key) s_hit[ot] = make_float4(t, u, v, __int_as_float((int)id));
+        __syncwarp();
+      }
+      if (take) {
+        if (s_key[tid] != ~0ull) best_t = s_hit[tid].x;
+        cnt -= take;
+        beg += take;
+        if (cnt == 0 && !pop()) fin = true;
+      }
     }
+
+    // ---- finished rays ----------------------------------------------------
+    if (fin) {
+      // IsInShadow form: closest hit && t < distance; closest: hits at or
+      // beyond the ray's tmax are reported as misses.
+      const float4 h = s_hit[tid];
+      const int id = lost ? -1 : __float_as_int(h.w);
+      const bool hit = id >= 0 && h.x < s_lim[tid].y;
+      if (ANY) {
+        reinterpret_cast<uint8_t*>(P.out)[ray] = hit ? 1 : 0;
+      } else {
+        reinterpret_cast<int4*>(P.out)[ray] =
+            hit ? make_int4(id, __float_as_int(h.x), __float_as_int(h.y), __float_as_int(h.z))
+                : make_int4(-1, 0, 0, 0);
+      }
+      active = false;
+      node = 0;
+      cnt = 0;
+    }
+    __syncwarp();
   }
 }
 
@@ -1201,18 +1348,18 @@ int launch_kd(const DevAccel& a, const float* rays, size_t n, void* out, cudaStr
     p.lo[i] = a.kd_root_lo[i];
     p.hi[i] = a.kd_root_hi[i];
   }
-  int grid = device_sm_count(a.device) * kKdBlocks;
-  unsigned need = (unsigned)((n + 127) / 128);
-  if ((unsigned)grid > need) grid = (int)need;
-  if (grid < 1) grid = 1;
-  const bool small = a.tree_depth > 0 && a.tree_depth <= 32;
-  if (a.predicate == ENC_PRED_REFERENCE) {
-    if (small) kd_trace<true, ANY, 32><<<grid, 128, 0, s>>>(p);
-    else kd_trace<true, ANY, 64><<<grid, 128, 0, s>>>(p);
-  } else {
-    if (small) kd_trace<false, ANY, 32><<<grid, 128, 0, s>>>(p);
-    else kd_trace<false, ANY, 64><<<grid, 128, 0, s>>>(p);
+  const uint32_t slot =
+      __atomic_fetch_add(const_cast<uint32_t*>(&a.counter_seq), 1u, __ATOMIC_RELAXED) % kQueueSlots;
+  p.counter = a.d_counter + slot;
+  const int sms = device_sm_count(a.device);
+  int grid = sms * kKdBlocks;
+  p.share = ray_share(Launch(), n, sms, &grid);
+  if (p.share == 0) {
+    cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return (int)e;
   }
+  if (a.predicate == ENC_PRED_REFERENCE) kd_trace<true, ANY><<<grid, 128, 0, s>>>(p);
+  else kd_trace<false, ANY><<<grid, 128, 0, s>>>(p);
   return (int)cudaGetLastError();
 }
 
