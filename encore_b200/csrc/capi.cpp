@@ -19,7 +19,9 @@
 struct enc_accel_s {
   enc::DevAccel dev;
   enc::WaveScratch wave;  // photon tracer scratch
-  enc::WBVHHost host;  // wide BVH kept on the host for refits
+  enc::WBVHHost host;  // wide BVH kept on the host for refits (its tree; a device refit
+                       // leaves the boxes here as they were)
+  enc::RefitScratch refit;
   std::mutex mu;  // serialises the host-buffer forms (shared staging buffers)
   void* d_stage_in = nullptr;
   void* d_stage_out = nullptr;
@@ -360,7 +362,21 @@ enc_status enc_accel_refit(enc_accel a, const float* tri_verts, uint32_t ntris) 
   DeviceScope ds(d.device);
   double t0 = now_s();
   try {
+    bool done = false;
     if (d.kind == ENC_ACCEL_WBVH) {
+      float lo[3], hi[3];
+      const int re = refit_device(d, a->host, &a->refit, tri_verts, lo, hi, &done);
+      if (re != 0) return cuda_fail((cudaError_t)re, "device refit");
+      if (done) {
+        for (int i = 0; i < 3; ++i) {
+          d.lo[i] = a->host.lo[i] = lo[i];
+          d.hi[i] = a->host.hi[i] = hi[i];
+        }
+      }
+    }
+    if (done) {
+      // nodes and triangles are in place
+    } else if (d.kind == ENC_ACCEL_WBVH) {
       refit_wbvh(&a->host, tri_verts, ntris);
       ENC_CUDA(cudaMemcpy(d.d_nodes, a->host.nodes.data(), a->host.nodes.size(), cudaMemcpyHostToDevice),
                "refit upload");
@@ -624,6 +640,7 @@ enc_status enc_accel_destroy(enc_accel a) {
   DeviceScope ds(a->dev.device);
   free_dev(a->dev);
   free_wave_scratch(&a->wave);
+  free_refit_scratch(&a->refit);
   cudaFree(a->d_stage_in);
   cudaFree(a->d_stage_od);
   cudaFree(a->d_stage_out);

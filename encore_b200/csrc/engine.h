@@ -162,6 +162,31 @@ void build_kd_reference(const float* tri_verts, uint32_t ntris, KdHost* out);
 // same tree shape) and rewrites its triangle records.
 void refit_wbvh(WBVHHost* h, const float* tri_verts, uint32_t ntris);
 void make_dev_tris(const float* tri_verts, uint32_t ntris, const uint32_t* order, DevTri* out);
+// How far triangle boxes are padded in a scene of these bounds: 1e-5 of the
+// larger of its extent and its largest coordinate.
+float box_pad(const float lo[3], const float hi[3], float maxabs);
+// The node ranges of the tree's levels (level l: [start[l], start[l + 1])).
+// False for a table that no builder writes: a level out of order, a child that
+// does not follow its parent, a node reached twice or never, an empty node, an
+// index out of range.
+bool refit_levels_of(const WBVHHost& h, std::vector<uint32_t>& start);
+
+// Device refit (refit.cu): its scratch, kept with the accelerator once it has
+// been refitted, and the tree's levels.
+struct RefitScratch {
+  void* mem = nullptr;
+  size_t bytes = 0;
+  bool planned = false, usable = false;
+  std::vector<uint32_t> level_start;
+};
+void free_refit_scratch(RefitScratch* r);
+// Refits `d` (a wide BVH whose tree is `host`) in place; lo, hi: the scene's
+// new bounds.  *done = false with status 0: nothing was changed, and the host
+// refit has to do it (a table refit_levels_of refuses, a coordinate that is not
+// finite or too large for a grid, no memory for the scratch).  Returns a CUDA
+// error code; `d.device` must be current.
+int refit_device(const DevAccel& d, const WBVHHost& host, RefitScratch* r, const float* tri_verts,
+                 float lo[3], float hi[3], bool* done);
 
 // Launch parameters after defaults are applied.
 struct Launch {

@@ -390,6 +390,12 @@ void make_dev_tris(const float* v, uint32_t n, const uint32_t* order, DevTri* ou
   }
 }
 
+float box_pad(const float lo[3], const float hi[3], float maxabs) {
+  const float ext = std::max(std::max(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
+  const float pad = 1e-5f * std::max(ext, maxabs);
+  return pad > 0.f ? pad : 1e-30f;
+}
+
 namespace {
 
 // Triangle boxes padded by 1e-5 of the larger of the scene extent and the
@@ -412,10 +418,7 @@ std::vector<Box> padded_boxes(const float* v, uint32_t n, float lo[3], float hi[
     scene.grow(b);
     for (int k = 0; k < 9; ++k) maxabs = std::max(maxabs, std::fabs(t[k]));
   }
-  const float ext = std::max(std::max(scene.hi[0] - scene.lo[0], scene.hi[1] - scene.lo[1]),
-                             scene.hi[2] - scene.lo[2]);
-  float pad = 1e-5f * std::max(ext, maxabs);
-  if (!(pad > 0.f)) pad = 1e-30f;
+  const float pad = box_pad(scene.lo, scene.hi, maxabs);
   if (cent) cent->resize(3 * (size_t)n);
   for (uint32_t i = 0; i < n; ++i)
     for (int a = 0; a < 3; ++a) {
@@ -479,6 +482,50 @@ void refit_wbvh(WBVHHost* h, const float* tri_verts, uint32_t ntris) {
   if (h->width == 2) refit_w<2>(h, tri_verts, ntris);
   else if (h->width == 4) refit_w<4>(h, tri_verts, ntris);
   else refit_w<8>(h, tri_verts, ntris);
+}
+
+namespace {
+
+template <int W>
+bool levels_w(const WBVHHost& h, std::vector<uint32_t>& start) {
+  using L = WNodeLayout<W>;
+  if (h.nnodes == 0 || h.nodes.size() != (size_t)h.nnodes * L::kBytes) return false;
+  start.assign(1, 0);
+  uint64_t next = 1;        // the first node not yet reached as a child
+  uint32_t level_end = 1;   // end of the level that node i lies in
+  for (uint32_t i = 0; i < h.nnodes; ++i) {
+    if (i == level_end) {
+      if (next <= level_end) return false;  // nodes that no node leads to
+      start.push_back(level_end);
+      level_end = (uint32_t)next;
+    }
+    const uint8_t* raw = h.nodes.data() + (size_t)i * L::kBytes;
+    WNodeHeader hd;
+    std::memcpy(&hd, raw, sizeof(hd));
+    uint32_t rank = 0;
+    bool any = false;
+    for (int c = 0; c < W; ++c) {
+      const uint32_t m = raw[L::kMetaOff + c];
+      if (m == 0) continue;
+      any = true;
+      if (m < 32) {
+        if (m != ++rank || hd.child_base + (uint64_t)(m - 1) != next) return false;
+        if (++next > h.nnodes) return false;
+      } else if ((uint64_t)hd.tri_base + (m & 31u) + (m >> 5) > h.tri_order.size()) {
+        return false;
+      }
+    }
+    if (!any) return false;
+  }
+  start.push_back(level_end);
+  return next == h.nnodes && level_end == h.nnodes && start.size() <= 65;
+}
+
+}  // namespace
+
+bool refit_levels_of(const WBVHHost& h, std::vector<uint32_t>& start) {
+  return h.width == 2 ? levels_w<2>(h, start)
+                      : (h.width == 4 ? levels_w<4>(h, start) : levels_w<8>(h, start));
 }
 
 void build_wbvh(const float* tri_verts, uint32_t ntris, int width, int max_leaf, WBVHHost* out) {
