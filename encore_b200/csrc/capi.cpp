@@ -1045,6 +1045,151 @@ enc_status enc_accel_count_visits(enc_accel a, const float* d_rays, size_t nrays
 // ---------------------------------------------------------------------------
 // PhotonMap
 
+namespace {
+
+// Up to this many photons a map is built on the host, where the device build's
+// launches take longer: 436 / 497 / 641 / 849 us on the host for 100 / 1,000 /
+// 2,000 / 4,000 photons, 471 / 512 / 544 / 567 us on the device.
+constexpr size_t kHostPhotons = 1024;
+
+// One allocation for a map's arrays, whose sizes photon_layout or a file
+// header has set, and for the device build's scratch (a cudaMalloc and a
+// cudaFree take about 0.3 ms each, as long as building 100,000 photons); the
+// status word starts at 0.
+cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  const size_t o_status = up(kGatherSlots * 4), o_box = o_status + 256,
+               o_leaf = o_box + up(4 * d.box_floats), o_pos = o_leaf + up(4 * d.leaf_words),
+               rec = 16 * (size_t)d.n;
+  const size_t o_build = o_pos + up(3 * rec);
+  cudaError_t e = cudaMalloc(&d.slab, o_build + scratch + 256);
+  if (e != cudaSuccess) {
+    d.slab = nullptr;
+    return e;
+  }
+  char* base = static_cast<char*>(d.slab);
+  d.d_counter = reinterpret_cast<uint32_t*>(base);
+  d.d_status = reinterpret_cast<uint32_t*>(base + o_status);
+  d.d_box = reinterpret_cast<float*>(base + o_box);
+  d.d_leaf = reinterpret_cast<uint32_t*>(base + o_leaf);
+  d.d_pos4 = reinterpret_cast<float*>(base + o_pos);
+  d.d_nrm4 = reinterpret_cast<float*>(base + o_pos + rec);
+  d.d_pow4 = reinterpret_cast<float*>(base + o_pos + 2 * rec);
+  d.build = scratch ? base + o_build : nullptr;
+  return cudaMemset(d.d_status, 0, 16);
+}
+
+// Whether kernels on `device` can read bytes at p: inside one of its own
+// allocations.  (A copy checks that by itself; a kernel would fault.)
+bool readable_on(const void* p, size_t bytes, int device) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != device ||
+      (reinterpret_cast<uintptr_t>(p) & 3u) != 0)
+    return false;
+  typedef int (*Range)(unsigned long long*, size_t*, unsigned long long);
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+  if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &found) !=
+          cudaSuccess ||
+      found != cudaDriverEntryPointSuccess || !fn) {
+    cudaGetLastError();
+    return false;
+  }
+  unsigned long long lo = 0;
+  size_t size = 0;
+  const unsigned long long a = (unsigned long long)reinterpret_cast<uintptr_t>(p);
+  return reinterpret_cast<Range>(fn)(&lo, &size, a) == 0 && a >= lo && a - lo <= size &&
+         bytes <= size - (a - lo);
+}
+
+// The map's arrays from a host build.
+cudaError_t host_photon_map(const float* pos, const float* normal, const float* power,
+                            DevPhotonMap& d, const char* what) {
+  try {
+    PhotonHost h;
+    build_photon_tree(pos, normal, power, d.n, &h);
+    const void* src[5] = {h.box.data(), h.leaf.data(), h.pos4.data(), h.nrm4.data(), h.pow4.data()};
+    void* dst[5] = {d.d_box, d.d_leaf, d.d_pos4, d.d_nrm4, d.d_pow4};
+    const size_t words[5] = {h.box.size(), h.leaf.size(), h.pos4.size(), h.nrm4.size(),
+                             h.pow4.size()};
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < 5 && e == cudaSuccess; ++i)
+      if (words[i]) e = cudaMemcpy(dst[i], src[i], 4 * words[i], cudaMemcpyHostToDevice);
+    return e;
+  } catch (const std::exception& ex) {
+    set_error(std::string(what) + ": " + ex.what());
+    return cudaErrorMemoryAllocation;
+  }
+}
+
+// A map over n photons whose three arrays lie in device memory (`on_device`)
+// or in host memory.
+enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, int32_t caustic,
+                           int32_t device, enc_photonmap* out, const char* what) {
+  enc_photonmap m = new (std::nothrow) enc_photonmap_s();
+  if (!m) return ENC_ERR_OUT_OF_MEMORY;
+  DevPhotonMap& d = m->dev;
+  d.caustic = caustic ? 1 : 0;
+  d.device = device;
+  photon_layout(n, &d);
+  const size_t bytes = 12 * n;
+  bool build = n > kHostPhotons;
+  cudaError_t e = alloc_photon_map(d, build ? photon_build_scratch(n) : 0);
+  if (e == cudaErrorMemoryAllocation && build) {  // the host build needs no scratch
+    cudaGetLastError();
+    build = false;
+    e = alloc_photon_map(d, 0);
+  }
+  // Photons that a kernel cannot read where they are get copied for the build;
+  // without room for the copy the host builds the map.
+  bool direct = on_device && build;
+  for (int i = 0; i < 3 && direct; ++i) direct = readable_on(src[i], bytes, device);
+  void* work = nullptr;
+  if (e == cudaSuccess && build && !direct && cudaMalloc(&work, 3 * bytes) != cudaSuccess) {
+    cudaGetLastError();
+    work = nullptr;
+    build = false;
+  }
+  if (e == cudaSuccess && build) {
+    const float* in[3] = {src[0], src[1], src[2]};
+    for (int i = 0; i < 3 && e == cudaSuccess && !direct; ++i) {
+      float* to = static_cast<float*>(work) + 3 * n * i;
+      e = cudaMemcpy(to, src[i], bytes,
+                     on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
+      in[i] = to;
+    }
+    if (e == cudaSuccess)
+      e = (cudaError_t)build_photon_device(in[0], in[1], in[2], d, d.build);
+  } else if (e == cudaSuccess && on_device) {
+    try {
+      std::vector<float> h[3];
+      for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
+        h[i].resize(3 * n);
+        if (n) e = cudaMemcpy(h[i].data(), src[i], bytes, cudaMemcpyDeviceToHost);
+      }
+      if (e == cudaSuccess) e = host_photon_map(h[0].data(), h[1].data(), h[2].data(), d, what);
+    } catch (const std::exception&) {
+      e = cudaErrorMemoryAllocation;
+    }
+  } else if (e == cudaSuccess) {
+    e = host_photon_map(src[0], src[1], src[2], d, what);
+  }
+  cudaFree(work);
+  if (e != cudaSuccess) {
+    cudaFree(d.slab);
+    delete m;
+    return cuda_fail(e, what);
+  }
+  *out = m;
+  return ENC_OK;
+}
+
+}  // namespace
+
 enc_status enc_photonmap_create(const float* pos, const float* normal, const float* power,
                                 size_t n, int32_t caustic, int32_t device, enc_photonmap* out) {
   if (!out || (n && (!pos || !normal || !power))) {
@@ -1062,51 +1207,8 @@ enc_status enc_photonmap_create(const float* pos, const float* normal, const flo
     return ENC_ERR_INVALID_ARG;
   }
   DeviceScope ds(device);
-  enc_photonmap m = new (std::nothrow) enc_photonmap_s();
-  if (!m) return ENC_ERR_OUT_OF_MEMORY;
-  DevPhotonMap& d = m->dev;
-  d.caustic = caustic ? 1 : 0;
-  d.device = device;
-  d.n = (uint32_t)n;
-  cudaError_t e = cudaSuccess;
-  try {
-    PhotonHost h;
-    build_photon_tree(pos, normal, power, n, &h);
-    d.nnodes = (uint32_t)h.nodes.size();
-    d.depth = h.depth;
-    d.nlevels = h.nlevels;
-    for (int l = 0; l < kPhotonMaxLevels; ++l) {
-      d.lvl_count[l] = h.lvl_count[l];
-      d.lvl_off[l] = h.lvl_off[l];
-      d.lvl_pad[l] = h.lvl_pad[l];
-    }
-    d.box_floats = h.box.size();
-    d.leaf_words = h.leaf.size();
-    e = upload(&d.d_box, h.box.data(), h.box.size());
-    if (e == cudaSuccess) e = upload(&d.d_leaf, h.leaf.data(), h.leaf.size());
-    if (e == cudaSuccess) e = upload(&d.d_pos4, h.pos4.data(), h.pos4.size());
-    if (e == cudaSuccess) e = upload(&d.d_nrm4, h.nrm4.data(), h.nrm4.size());
-    if (e == cudaSuccess) e = upload(&d.d_pow4, h.pow4.data(), h.pow4.size());
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_status, 16);
-    if (e == cudaSuccess) e = cudaMemset(d.d_status, 0, 16);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_counter, kGatherSlots * sizeof(uint32_t));
-  } catch (const std::exception& ex) {
-    set_error(std::string("enc_photonmap_create: ") + ex.what());
-    e = cudaErrorMemoryAllocation;
-  }
-  if (e != cudaSuccess) {
-    cudaFree(d.d_box);
-    cudaFree(d.d_leaf);
-    cudaFree(d.d_pos4);
-    cudaFree(d.d_nrm4);
-    cudaFree(d.d_pow4);
-    cudaFree(d.d_status);
-    cudaFree(d.d_counter);
-    delete m;
-    return cuda_fail(e, "enc_photonmap_create");
-  }
-  *out = m;
-  return ENC_OK;
+  const float* src[3] = {pos, normal, power};
+  return make_photon_map(src, false, n, caustic, device, out, "enc_photonmap_create");
 }
 
 enc_status enc_photonmap_create_device(const float* d_pos, const float* d_nrm, const float* d_pow,
@@ -1116,16 +1218,19 @@ enc_status enc_photonmap_create_device(const float* d_pos, const float* d_nrm, c
     set_error("enc_photonmap_create_device: null argument");
     return ENC_ERR_INVALID_ARG;
   }
-  std::vector<float> pos(3 * n), nrm(3 * n), pw(3 * n);
-  {
-    DeviceScope ds(device);
-    if (n) {
-      ENC_CUDA(cudaMemcpy(pos.data(), d_pos, 12 * n, cudaMemcpyDeviceToHost), "D2H photons");
-      ENC_CUDA(cudaMemcpy(nrm.data(), d_nrm, 12 * n, cudaMemcpyDeviceToHost), "D2H photons");
-      ENC_CUDA(cudaMemcpy(pw.data(), d_pow, 12 * n, cudaMemcpyDeviceToHost), "D2H photons");
-    }
+  *out = nullptr;
+  if (n > 0x7fffffffull) {
+    set_error("enc_photonmap_create_device: too many photons");
+    return ENC_ERR_INVALID_ARG;
   }
-  return enc_photonmap_create(pos.data(), nrm.data(), pw.data(), n, caustic, device, out);
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
+    set_error("enc_photonmap_create_device: no such CUDA device");
+    return ENC_ERR_INVALID_ARG;
+  }
+  DeviceScope ds(device);
+  const float* src[3] = {d_pos, d_nrm, d_pow};
+  return make_photon_map(src, true, n, caustic, device, out, "enc_photonmap_create_device");
 }
 
 namespace {
@@ -1247,27 +1352,16 @@ enc_status enc_photonmap_deserialize(const void* buf, size_t size, int32_t devic
   d.box_floats = h.box_floats;
   d.leaf_words = h.leaf_words;
   const char* p = static_cast<const char*>(buf) + sizeof(h);
-  const float* fp = reinterpret_cast<const float*>(p);
-  cudaError_t e = upload(&d.d_box, fp, h.box_floats);
-  p += 4 * h.box_floats;
-  if (e == cudaSuccess) e = upload(&d.d_leaf, reinterpret_cast<const uint32_t*>(p), h.leaf_words);
-  p += 4 * h.leaf_words;
-  float** dst[3] = {&d.d_pos4, &d.d_nrm4, &d.d_pow4};
-  for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
-    e = upload(dst[i], reinterpret_cast<const float*>(p), 4 * (size_t)h.n);
-    p += 16 * (size_t)h.n;
+  cudaError_t e = alloc_photon_map(d, 0);
+  void* dst[5] = {d.d_box, d.d_leaf, d.d_pos4, d.d_nrm4, d.d_pow4};
+  const size_t bytes[5] = {4 * h.box_floats, 4 * h.leaf_words, 16 * (size_t)h.n,
+                           16 * (size_t)h.n, 16 * (size_t)h.n};
+  for (int i = 0; i < 5; ++i) {
+    if (e == cudaSuccess && bytes[i]) e = cudaMemcpy(dst[i], p, bytes[i], cudaMemcpyHostToDevice);
+    p += bytes[i];
   }
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_status, 16);
-  if (e == cudaSuccess) e = cudaMemset(d.d_status, 0, 16);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_counter, kGatherSlots * sizeof(uint32_t));
   if (e != cudaSuccess) {
-    cudaFree(d.d_box);
-    cudaFree(d.d_leaf);
-    cudaFree(d.d_pos4);
-    cudaFree(d.d_nrm4);
-    cudaFree(d.d_pow4);
-    cudaFree(d.d_status);
-    cudaFree(d.d_counter);
+    cudaFree(d.slab);
     delete m;
     return cuda_fail(e, "enc_photonmap_deserialize");
   }
@@ -1278,13 +1372,7 @@ enc_status enc_photonmap_deserialize(const void* buf, size_t size, int32_t devic
 enc_status enc_photonmap_destroy(enc_photonmap m) {
   if (!m) return ENC_OK;
   DeviceScope ds(m->dev.device);
-  cudaFree(m->dev.d_box);
-  cudaFree(m->dev.d_leaf);
-  cudaFree(m->dev.d_pos4);
-  cudaFree(m->dev.d_nrm4);
-  cudaFree(m->dev.d_pow4);
-  cudaFree(m->dev.d_status);
-  cudaFree(m->dev.d_counter);
+  cudaFree(m->dev.slab);
   cudaFree(m->d_stage);
   delete m;
   return ENC_OK;

@@ -62,6 +62,28 @@ struct TreeBuilder {
 
 }  // namespace
 
+void photon_layout(size_t n, DevPhotonMap* d) {
+  int depth = 0;
+  while (((n + ((size_t)1 << depth) - 1) >> depth) > (size_t)kPhotonLeaf) ++depth;
+  d->n = (uint32_t)n;
+  d->depth = depth;
+  d->nnodes = (uint32_t)(((size_t)2 << depth) - 1);
+  d->nlevels = 0;
+  d->box_floats = 0;
+  size_t count = (size_t)1 << depth;
+  d->leaf_words = 2 * count;
+  for (;;) {
+    const size_t pad = (count + 31) / 32 * 32;
+    const int l = d->nlevels++;
+    d->lvl_count[l] = (uint32_t)count;
+    d->lvl_pad[l] = (uint32_t)pad;
+    d->lvl_off[l] = (uint32_t)d->box_floats;
+    d->box_floats += 6 * pad;
+    if (count <= 32) break;
+    count = (count + 31) / 32;
+  }
+}
+
 void build_photon_tree(const float* pos, const float* nrm, const float* power, size_t n,
                        PhotonHost* out) {
   if (n > 0x7fffffffu) throw std::runtime_error("too many photons");

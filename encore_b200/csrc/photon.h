@@ -54,13 +54,15 @@ void build_photon_tree(const float* pos, const float* nrm, const float* power, s
 constexpr int kGatherSlots = 256;
 
 struct DevPhotonMap {
+  void* slab = nullptr;        // the one allocation every array below lies in
+  void* build = nullptr;       // ... and the device build's scratch, if it has that
   float* d_box = nullptr;      // PhotonHost::box
   uint32_t* d_leaf = nullptr;  // PhotonHost::leaf
   int nlevels = 0;
   uint32_t lvl_count[kPhotonMaxLevels] = {};
   uint32_t lvl_off[kPhotonMaxLevels] = {};
   uint32_t lvl_pad[kPhotonMaxLevels] = {};
-  float* d_pos4 = nullptr;
+  float* d_pos4 = nullptr;  // pos4, nrm4 and pow4 lie back to back
   float* d_nrm4 = nullptr;
   float* d_pow4 = nullptr;
   uint32_t* d_status = nullptr;
@@ -77,6 +79,18 @@ struct DevPhotonMap {
   size_t box_floats = 0;   // PhotonHost::box.size()
   size_t leaf_words = 0;   // PhotonHost::leaf.size()
 };
+
+// Fills depth, nnodes, the levels, box_floats and leaf_words of a map of n photons
+// (n <= 2^31 - 1) as build_photon_tree lays it out.
+void photon_layout(size_t n, DevPhotonMap* d);
+
+// Device build (photon_build.cu) of a map whose arrays are allocated, from
+// n >= 1 photons in device memory (3 floats each per photon, outside the map's
+// arrays).  `scratch`: photon_build_scratch(n) bytes, 256-byte aligned.  On the legacy default stream; waits for it.
+// Returns a CUDA error code; d.device must be current.
+size_t photon_build_scratch(size_t n);
+int build_photon_device(const float* d_pos, const float* d_nrm, const float* d_pow,
+                        const DevPhotonMap& d, void* scratch);
 
 // Launchers (gather.cu).  k <= 256.  Asynchronous on `stream`.
 int launch_radiance(const DevPhotonMap& m, const float* d_qpos, const float* d_qnrm, size_t nq,
