@@ -76,11 +76,55 @@ enc_status cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
 
+// Memory of photon maps.  A renderer makes a map per frame, and a cudaMalloc
+// and a cudaFree take about 0.35 and 0.3 ms (several times that on a busy host),
+// a third of making and using a map of 500,000 photons; so a map's allocation
+// comes from a pool per device that keeps up to kPoolKeep bytes of freed maps.
+// The kept memory goes back to the device when an accelerator on it is
+// destroyed and when an allocation of this library does not fit.  The pool
+// itself serialises its callers.
+constexpr uint64_t kPoolKeep = 128ull << 20;
+constexpr int kPoolDevices = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kPoolDevices] = {};
+bool g_pool_tried[kPoolDevices] = {};
+
+// The device's pool; null where it has none (then maps use cudaMalloc).
+cudaMemPool_t map_pool(int device, bool create) {
+  if (device < 0 || device >= kPoolDevices) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool[device] && create && !g_pool_tried[device]) {
+    g_pool_tried[device] = true;
+    int can = 0;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kPoolKeep;
+    if (cudaDeviceGetAttribute(&can, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess &&
+        can && cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+      if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+        g_pool[device] = pool;
+      else
+        cudaMemPoolDestroy(pool);
+    }
+    cudaGetLastError();
+  }
+  return g_pool[device];
+}
+
+// Gives the device back what its pool keeps.
+void trim_map_pool(int device) {
+  if (cudaMemPool_t pool = map_pool(device, false)) cudaMemPoolTrimTo(pool, 0);
+}
+
 template <class T>
 cudaError_t upload(T** dst, const T* src, size_t count) {
   *dst = nullptr;
   if (count == 0) return cudaSuccess;
-  cudaError_t e = cudaMalloc((void**)dst, count * sizeof(T));
+  cudaError_t e = device_malloc((void**)dst, count * sizeof(T));
   if (e != cudaSuccess) return e;
   return cudaMemcpy(*dst, src, count * sizeof(T), cudaMemcpyHostToDevice);
 }
@@ -108,7 +152,7 @@ enc_status grow(void** p, size_t* cap, size_t need) {
   *p = nullptr;
   *cap = 0;
   size_t n = need + need / 4;
-  cudaError_t e = cudaMalloc(p, n);
+  cudaError_t e = device_malloc(p, n);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(staging)");
   *cap = n;
   return ENC_OK;
@@ -130,6 +174,19 @@ enc_status read_status(enc_accel a, cudaStream_t s) {
 }  // namespace
 
 void set_error(const std::string& msg) { g_err = msg; }
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  int device = -1;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess &&
+      map_pool(device, false)) {
+    cudaGetLastError();
+    cudaDeviceSynchronize();  // maps freed in stream order become the pool's to give back
+    trim_map_pool(device);
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
 
 const DevAccel* accel_device_view(enc_accel a) { return a ? &a->dev : nullptr; }
 
@@ -651,6 +708,7 @@ enc_status enc_accel_destroy(enc_accel a) {
   for (cudaEvent_t e : a->ev_wide) cudaEventDestroy(e);
   if (a->pipe_start) cudaEventDestroy(a->pipe_start);
   if (a->pipe_done) cudaEventDestroy(a->pipe_done);
+  trim_map_pool(a->dev.device);
   delete a;
   return ENC_OK;
 }
@@ -1053,19 +1111,26 @@ namespace {
 constexpr size_t kHostPhotons = 1024;
 
 // One allocation for a map's arrays, whose sizes photon_layout or a file
-// header has set, and for the device build's scratch (a cudaMalloc and a
-// cudaFree take about 0.3 ms each, as long as building 100,000 photons); the
-// status word starts at 0.
+// header has set, and for the device build's scratch; the status word starts
+// at 0.
 cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   const size_t o_status = up(kGatherSlots * 4), o_box = o_status + 256,
                o_leaf = o_box + up(4 * d.box_floats), o_pos = o_leaf + up(4 * d.leaf_words),
                rec = 16 * (size_t)d.n;
   const size_t o_build = o_pos + up(3 * rec);
-  cudaError_t e = cudaMalloc(&d.slab, o_build + scratch + 256);
-  if (e != cudaSuccess) {
-    d.slab = nullptr;
-    return e;
+  const size_t bytes = o_build + scratch + 256;
+  cudaMemPool_t pool = map_pool(d.device, true);
+  // on the legacy default stream, where the map is then written; its creation
+  // waits for that, so the map may be used on any stream
+  d.pooled = pool && cudaMallocFromPoolAsync(&d.slab, bytes, pool, 0) == cudaSuccess;
+  if (!d.pooled) {
+    cudaGetLastError();
+    cudaError_t e = device_malloc(&d.slab, bytes);
+    if (e != cudaSuccess) {
+      d.slab = nullptr;
+      return e;
+    }
   }
   char* base = static_cast<char*>(d.slab);
   d.d_counter = reinterpret_cast<uint32_t*>(base);
@@ -1077,6 +1142,18 @@ cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
   d.d_pow4 = reinterpret_cast<float*>(base + o_pos + 2 * rec);
   d.build = scratch ? base + o_build : nullptr;
   return cudaMemset(d.d_status, 0, 16);
+}
+
+// A map may still be read on any stream of its device when it is destroyed;
+// cudaFree waits for them by itself.
+void free_photon_map(DevPhotonMap& d) {
+  if (d.pooled) {
+    cudaDeviceSynchronize();
+    cudaFreeAsync(d.slab, 0);
+  } else {
+    cudaFree(d.slab);
+  }
+  d.slab = nullptr;
 }
 
 // Whether kernels on `device` can read bytes at p: inside one of its own
@@ -1149,7 +1226,7 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   bool direct = on_device && build;
   for (int i = 0; i < 3 && direct; ++i) direct = readable_on(src[i], bytes, device);
   void* work = nullptr;
-  if (e == cudaSuccess && build && !direct && cudaMalloc(&work, 3 * bytes) != cudaSuccess) {
+  if (e == cudaSuccess && build && !direct && device_malloc(&work, 3 * bytes) != cudaSuccess) {
     cudaGetLastError();
     work = nullptr;
     build = false;
@@ -1180,7 +1257,7 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   }
   cudaFree(work);
   if (e != cudaSuccess) {
-    cudaFree(d.slab);
+    free_photon_map(d);
     delete m;
     return cuda_fail(e, what);
   }
@@ -1361,7 +1438,7 @@ enc_status enc_photonmap_deserialize(const void* buf, size_t size, int32_t devic
     p += bytes[i];
   }
   if (e != cudaSuccess) {
-    cudaFree(d.slab);
+    free_photon_map(d);
     delete m;
     return cuda_fail(e, "enc_photonmap_deserialize");
   }
@@ -1372,7 +1449,7 @@ enc_status enc_photonmap_deserialize(const void* buf, size_t size, int32_t devic
 enc_status enc_photonmap_destroy(enc_photonmap m) {
   if (!m) return ENC_OK;
   DeviceScope ds(m->dev.device);
-  cudaFree(m->dev.slab);
+  free_photon_map(m->dev);
   cudaFree(m->d_stage);
   delete m;
   return ENC_OK;

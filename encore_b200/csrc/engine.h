@@ -9,6 +9,8 @@
 #include <string>
 #include <vector>
 
+#include <cuda_runtime_api.h>
+
 #include "../../include/encore_b200.h"
 
 namespace enc {
@@ -256,6 +258,10 @@ int launch_multi_closest(const MultiLaunch& m, const Launch& L, void* stream);
 // Any hit (uint8 occluded per ray) for every batch of the table.
 int launch_multi_any(const MultiLaunch& m, const Launch& L, void* stream);
 int device_sm_count(int device);
+
+// cudaMalloc on the current device; if that does not fit, once more after the
+// memory kept for photon maps has been given back (capi.cpp).
+cudaError_t device_malloc(void** p, size_t bytes);
 
 // Error reporting (capi.cpp).
 void set_error(const std::string& msg);

@@ -55,6 +55,7 @@ constexpr int kGatherSlots = 256;
 
 struct DevPhotonMap {
   void* slab = nullptr;        // the one allocation every array below lies in
+  bool pooled = false;         // it came from the device's pool of map memory
   void* build = nullptr;       // ... and the device build's scratch, if it has that
   float* d_box = nullptr;      // PhotonHost::box
   uint32_t* d_leaf = nullptr;  // PhotonHost::leaf

@@ -21,7 +21,7 @@
 //
 // What bounds it: some 65 short launches (three per level) of a few
 // microseconds, each streaming 4 to 24 bytes per photon and axis through L2.
-// 500,000 photons: 44.9 ms on the host, about 1 ms here, 0.3 of it the allocation.
+// 500,000 photons: 44.9 ms on the host, 0.63 ms here.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -268,7 +268,7 @@ int refit_device(const DevAccel& d, const WBVHHost& host, RefitScratch* r, const
   const size_t need = o_out + 256;
   if (r->bytes < need) {
     free_refit_scratch(r);
-    if (cudaMalloc(&r->mem, need) != cudaSuccess) {
+    if (device_malloc(&r->mem, need) != cudaSuccess) {
       cudaGetLastError();  // no room for the scratch: the host refit needs none
       r->mem = nullptr;
       return 0;

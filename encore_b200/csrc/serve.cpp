@@ -346,18 +346,18 @@ enc_status enc_server_create(const enc_server_opts* opts, enc_server* out) {
   int prev = -1;
   cudaGetDevice(&prev);
   cudaSetDevice(o.device);
-  cudaError_t e = cudaMalloc((void**)&S->d_scenes, kMaxScenes * sizeof(SceneDesc));
+  cudaError_t e = device_malloc((void**)&S->d_scenes, kMaxScenes * sizeof(SceneDesc));
   S->slots.resize(o.slots);
   for (Slot& sl : S->slots) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sl.s, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&sl.d_rays, o.slot_rays * 32);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&sl.d_out, o.slot_rays * 16);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&sl.d_tab, 2 * kMaxReqPerSlot * sizeof(BatchDesc));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&sl.d_starts, 2 * (kMaxReqPerSlot + 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&sl.d_words, 16);
+    if (e == cudaSuccess) e = device_malloc((void**)&sl.d_rays, o.slot_rays * 32);
+    if (e == cudaSuccess) e = device_malloc((void**)&sl.d_out, o.slot_rays * 16);
+    if (e == cudaSuccess) e = device_malloc((void**)&sl.d_tab, 2 * kMaxReqPerSlot * sizeof(BatchDesc));
+    if (e == cudaSuccess) e = device_malloc((void**)&sl.d_starts, 2 * (kMaxReqPerSlot + 1) * 4);
+    if (e == cudaSuccess) e = device_malloc((void**)&sl.d_words, 16);
     if (e == cudaSuccess) e = cudaMemset(sl.d_words, 0, 16);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&sl.d_bstat, 2 * kMaxReqPerSlot * 4);
+    if (e == cudaSuccess) e = device_malloc((void**)&sl.d_bstat, 2 * kMaxReqPerSlot * 4);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&sl.h_tab, 2 * kMaxReqPerSlot * sizeof(BatchDesc));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&sl.h_starts, 2 * (kMaxReqPerSlot + 1) * 4);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&sl.h_bstat, 2 * kMaxReqPerSlot * 4);

@@ -509,13 +509,13 @@ enc_status trace_photons(enc_accel accel, const enc_photon_opts* o, int split, f
     // grow the kept scratch (no allocation once it is large enough)
     free_wave_scratch(&w);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
-      e = cudaMalloc((void**)&w.rays[i], n * 32);
-      if (e == cudaSuccess) e = cudaMalloc((void**)&w.path[i], n * 4);
-      if (e == cudaSuccess) e = cudaMalloc((void**)&w.srays[i], n * 32);
-      if (e == cudaSuccess) e = cudaMalloc((void**)&w.spath[i], n * 4);
+      e = device_malloc((void**)&w.rays[i], n * 32);
+      if (e == cudaSuccess) e = device_malloc((void**)&w.path[i], n * 4);
+      if (e == cudaSuccess) e = device_malloc((void**)&w.srays[i], n * 32);
+      if (e == cudaSuccess) e = device_malloc((void**)&w.spath[i], n * 4);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&w.hits, n * 16);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&w.counters, 32);
+    if (e == cudaSuccess) e = device_malloc(&w.hits, n * 16);
+    if (e == cudaSuccess) e = device_malloc((void**)&w.counters, 32);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&w.h_counts, 32);
     if (e != cudaSuccess) {
       free_wave_scratch(&w);
@@ -676,7 +676,7 @@ enc_status enc_photons_trace_maps(enc_accel accel, const enc_photon_opts* o, flo
   for (int m = 0; m < 2 && e == cudaSuccess; ++m) {
     const size_t cap = hs[m]->capacity;
     const size_t bytes = cap * (36 + (hs[m]->d_tag ? 4 : 0)) + 16;
-    e = cudaMalloc(&blocks[m], bytes);
+    e = device_malloc(&blocks[m], bytes);
     float* base = static_cast<float*>(blocks[m]);
     ds[m] = PhotonStore{base, base + 3 * cap, base + 6 * cap,
                         hs[m]->d_tag ? reinterpret_cast<uint32_t*>(base + 9 * cap) : nullptr,

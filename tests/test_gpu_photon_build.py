@@ -111,3 +111,73 @@ def test_nearest_and_radiance_match_the_oracle(gpu, n):
             near = ok[np.lexsort((ok, d[ok]))][:k]
             assert cnt[i] == len(near) and np.array_equal(idx[i, :cnt[i]], near)
             assert np.array_equal(d2[i, :cnt[i]], d[near])
+
+
+def test_memory_kept_for_maps_is_bounded_and_given_back(gpu):
+    """Freed maps leave at most the pool's bound behind, and nothing once an
+    accelerator on the device has been destroyed."""
+    import torch
+
+    from encore_b200 import Accelerator, scenes
+    small = scenes.random_triangles(64, seed=93, scale=1000.0)
+
+    def free_bytes():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    n = 3_000_000
+    d = [torch.rand(n, 3, device="cuda") for _ in range(3)]
+    for _ in range(2):  # the first pass also loads the kernels
+        Accelerator("wbvh").build(small).destroy()
+        before = free_bytes()
+        maps = [photon_map_from_device(*d, n) for _ in range(2)]
+        assert before - free_bytes() >= 2 * 48 * n
+        del maps
+        assert before - free_bytes() <= (128 << 20) + (64 << 20)
+        Accelerator("wbvh").build(small).destroy()
+        left = before - free_bytes()
+    assert left <= 4 << 20
+
+
+def test_maps_made_and_freed_by_several_threads(gpu):
+    """Threads that make, use and free maps at once, each on a stream of its
+    own, get the answers one thread gets alone."""
+    import threading
+
+    import torch
+    r = np.random.default_rng(94)
+    sizes = [1500, 20000, 70001, 150000]
+    sets = [photons("box", n) for n in sizes]
+    q = (r.random((4000, 3)) * [3.0, 1.0, 2.0]).astype(np.float32)
+    qn = np.eye(3, dtype=np.float32)[r.integers(0, 3, 4000)]
+    dq, dn = torch.from_numpy(q).cuda(), torch.from_numpy(qn).cuda()
+
+    def gather(i, stream):
+        d = [torch.from_numpy(x).cuda() for x in sets[i]]
+        torch.cuda.synchronize()
+        out = torch.zeros(4000, 3, device="cuda")
+        torch.cuda.synchronize()
+        pm = photon_map_from_device(*d, sizes[i])
+        pm.get_radiance_estimate_device(20, 0.3, dq, dn, 4000, out, stream=stream.cuda_stream)
+        del pm  # waits for the gather
+        return out.cpu().numpy()
+
+    want = [gather(i, torch.cuda.Stream()) for i in range(4)]
+    got, errors = {}, []
+
+    def work(i):
+        try:
+            s = torch.cuda.Stream()
+            got[i] = [gather(i, s) for _ in range(6)]
+        except Exception as e:  # noqa: BLE001 - reported below
+            errors.append(e)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for i in range(4):
+        for g in got[i]:
+            assert np.array_equal(g.view(np.int32), want[i].view(np.int32))
