@@ -214,6 +214,7 @@ struct BinSpec {
   float scale[3];  // cells per unit length on each axis
   float probe_len; // > 0: bin the point o + probe_len * d instead of o
   int bits[5];     // key bits: origin x, y, z, direction u, v
+  uint8_t place[5][kBinMaxDimBits];  // where each of them lies in the key
 };
 // Scratch layout: keys (n words), order (n words), histogram (2^key_bits
 // words), each 256-byte aligned.

@@ -152,3 +152,40 @@ def test_ordered_trace_skips_and_reports_entries_outside_the_batch(gpu, field):
     keep[7] = False
     assert np.array_equal(got[keep], want[keep])
     assert np.all(got[7] == -5)
+
+
+@pytest.mark.parametrize("cfg", [BinConfig(9, 0), BinConfig(18, 0)])
+@pytest.mark.parametrize("n,spread", [(1, 1.0), (511, 1.0), (512, 0.0), (513, 1.0), (60000, 0.001),
+                                      (60000, 1.0), (131073, 0.3)])
+def test_order_is_a_permutation_sorted_by_key(gpu, cfg, n, spread):
+    """The order itself, at the edges of a block's rays and from rays that all
+    share one bucket to rays spread over all of them."""
+    import torch
+    tris = scenes.random_triangles(500, seed=11, scale=1000.0)
+    acc = Accelerator("wbvh").build(tris)
+    info = acc.info()
+    lo, hi = (np.array(info[f], np.float32) for f in ("scene_lo", "scene_hi"))
+    rng = np.random.default_rng(12)
+    rays = scenes.random_sphere_rays(n, seed=13)
+    rays[:, 0:3] = lo + (hi - lo) * (0.4 + spread * (rng.random((n, 3)) - 0.4)).astype(np.float32)
+    d = torch.from_numpy(rays).cuda()
+    scratch = torch.empty(acc.bin_scratch_bytes(n, cfg), dtype=torch.uint8, device="cuda")
+    at = acc.bin_rays(d, n, scratch, cfg) - scratch.data_ptr()
+    torch.cuda.synchronize()
+    order = scratch[at:at + 4 * n].cpu().numpy().view(np.uint32)
+    assert np.array_equal(np.sort(order), np.arange(n))
+    # bits go to the axis with the widest cells first; interleaved from the top
+    bits, cell = [0, 0, 0], (hi - lo).copy()
+    for _ in range(cfg.origin_bits):
+        a = int(np.argmax(cell))
+        bits[a] += 1
+        cell[a] *= np.float32(0.5)
+    q = [np.clip((rays[:, a] - lo[a]) * np.float32(np.float32(1 << bits[a]) / (hi[a] - lo[a])), 0,
+                 (1 << bits[a]) - 1).astype(np.uint32) for a in range(3)]
+    key = np.zeros(n, np.uint32)
+    for level in range(9, -1, -1):
+        for a in range(3):
+            if level < bits[a]:
+                key = (key << 1) | ((q[a] >> level) & 1)
+    assert (np.diff(key[order].astype(np.int64)) >= 0).all()
+    acc.destroy()
