@@ -6,9 +6,9 @@
 //    the slowest ray of a batch).  The traversal stack lives in shared
 //    memory, one column per thread.  A visited node continues with its first
 //    hit internal child; the others stay on the stack as one group entry.
-//    The triangles of its hit leaves are tested in the same step: for closest
-//    hit by the whole warp together (all lanes' triangles, one per lane per
-//    round), for any hit and with LANE by each lane in turn.  Width 8 orders
+//    The triangles of its hit leaves are tested in the same step, by the whole
+//    warp together (all lanes' triangles, one per lane per round); with LANE by
+//    each lane in turn.  Width 8 orders
 //    children by octant (the builder places each child in the slot of its
 //    octant, so slot k ^ octm for k = 0..7 is roughly front to back for a ray
 //    with direction sign bits octm); widths 2 and 4 sort hit children by
@@ -40,9 +40,9 @@
 // 56 registers without spilling and ran 1.7 % faster than at 8 (64
 // registers) on the 2M-triangle heightfield workload; at 10 blocks (48
 // registers) it spills 42 bytes and lost 8 %.  The multi-scene form keeps 8
-// blocks: at 9 it spills 78 bytes.  The any-hit kernel keeps the per-lane
-// loop (its rays rarely reach a triangle before the first hit) at 9 blocks
-// (no spill; 3.9 % faster than 10 with a 28-byte spill).  The per-lane
+// blocks: at 9 it spills 78 bytes.  The any-hit kernel has no spill at 9
+// either; 1.5M shadow rays in 100,000 random triangles: 667 us, 665 at 8 and 715
+// at 10, and 4M over the heightfield 713, 737 and 744.  The per-lane
 // closest-hit form, which the host-buffer pipeline runs beside its copies,
 // keeps 10 (at 9 the pipeline measured about 1 % slower).
 constexpr int kBlocksClosest = 9;
@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   // Stack of node groups: one entry per visited node that still has hit
   // internal children, so the depth never exceeds the tree depth.
   //   W == 8: x = child_base, y = remaining hit children as bits k in
-  //           octant order (slot = k ^ octm) | internal-slot mask << 8;
+  //           octant order (slot = k ^ octm; any hit: slot = k) | internal-slot
+  //           mask << 8;
   //           lb = smallest entry distance among the group's hit children.
   //   W < 8:  x = child_base, y = ranks of the remaining children sorted by
   //           entry distance (3 bits each, nearest first) | count << 24;
@@ -305,9 +306,25 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   //   memory and leaves more of the SM's L1 to node and triangle loads.
   constexpr bool kCompact = W == 8;
   extern __shared__ uint2 s_stack[];
-  // Closest hit tests the triangles of the lanes' hit leaves as one warp
-  // (see below); any hit, and closest hit with LANE, keep one loop per lane.
-  constexpr bool kCoop = !ANY && !LANE;
+  // The triangles of the lanes' hit leaves are tested as one warp (see below);
+  // closest hit with LANE keeps one loop per lane.  Any hit, whose lanes wait
+  // for one another in that loop just the same: 811 -> 667 us for 1.5M shadow
+  // rays in 100,000 random triangles, half of them blocked, and 801 -> 713 us for
+  // 4M over the 2M-triangle heightfield, where few are.
+  constexpr bool kCoop = !LANE;
+  static_assert(!(ANY && LANE), "any hit has no per-lane form");
+  // Any hit stops at the first hit and culls nothing by distance, so its result
+  // does not depend on the order of the children; it takes them in slot order
+  // and saves the octant permutation (30,000 rays: 96 -> 88 us, 4M: 713 -> 701).
+  constexpr bool kOctants = !ANY;
+  // Idle lanes a warp waits for before it refills them.  A refill runs some 60
+  // instructions for the few lanes that ended in a step (three of 32, at ten
+  // visits per ray), so waiting for one more costs less than it saves.  At 1 / 2
+  // / 4 / 6 / 8 / 12: the heightfield's 4.18M rays 1,163 / 1,159 / 1,141 / 1,138 /
+  // 1,146 / 1,168 us, 1M eye rays on 10,000 triangles 344 / 343 / 342 / 346 / 353 /
+  // 371, 16 scenes in one launch 1,157 / 1,143 / 1,134 / 1,143 / 1,160 / 1,211, the
+  // shadow rays above 670 / 666 / 663 / 668 / 679 / 703.
+  constexpr int kRefill = LANE ? 1 : 4;
   // the per-lane form keeps the group bound (without it ptxas spills more)
   constexpr bool kBound = kGroupBound || LANE;
   // L2 priorities in the single-scene cooperative closest-hit form only: in
@@ -315,7 +332,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   // host-buffer pipeline runs, the evict_first hits left L2 before their copy
   // out (2 %); the multi-scene form, whose hits the server copies out after
   // each launch, keeps plain loads and stores too
-  constexpr bool kL2Hints = kCoop && !MULTI;
+  constexpr bool kL2Hints = kCoop && !MULTI && !ANY;
   __shared__ uint32_t s_coop_tri[kCoop ? 128 : 1];
   __shared__ uint32_t s_coop_own[kCoop ? 128 : 1];
   __shared__ unsigned long long s_coop_key[kCoop ? 128 : 1];
@@ -374,6 +391,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   while (true) {
     // ---- refill idle lanes from the warp pool --------------------------
     unsigned need = __ballot_sync(kFull, ray < 0);
+    if (__popc(need) < kRefill) need = 0;
     while (need && !exhausted) {
       if (pool_next >= pool_end) {
         if (!MULTI && P.share) {  // the warp's share is all it takes
@@ -634,9 +652,11 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
           }
           // hit internal children in octant order: bit k = slot k ^ voct
           uint32_t x = hm & imask;
-          if (voct & 1u) x = ((x & 0x55u) << 1) | ((x >> 1) & 0x55u);
-          if (voct & 2u) x = ((x & 0x33u) << 2) | ((x >> 2) & 0x33u);
-          if (voct & 4u) x = ((x & 0x0fu) << 4) | ((x >> 4) & 0x0fu);
+          if (kOctants) {
+            if (voct & 1u) x = ((x & 0x55u) << 1) | ((x >> 1) & 0x55u);
+            if (voct & 2u) x = ((x & 0x33u) << 2) | ((x >> 2) & 0x33u);
+            if (voct & 4u) x = ((x & 0x0fu) << 4) | ((x >> 4) & 0x0fu);
+          }
           hitk = x;
         } else {
 #pragma unroll
@@ -670,7 +690,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
           if (hitk) {
             const uint32_t imask = ew >> 24;
             const uint32_t k = __ffs(hitk) - 1;
-            const uint32_t slot = k ^ voct;
+            const uint32_t slot = kOctants ? k ^ voct : k;
             node = child_base + __popc(imask & ((1u << slot) - 1u));
             const uint32_t rest = hitk & (hitk - 1u);
             if (rest) {
@@ -735,12 +755,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
           float t, u, v;
           if (tri_test<CLAMP>(a, b, c, ox, oy, oz, dx, dy, dz, tmin, t, u, v)) {
             const int id = __float_as_int(c.y);
-            if (ANY) {
-              if (t < tmax) {
-                hit_any = true;
-                break;
-              }
-            } else if (t < best_t || (t == best_t && id < best_id)) {
+            if (t < best_t || (t == best_t && id < best_id)) {
               best_t = t;
               best_id = id;
               bu = u;
@@ -748,7 +763,6 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
             }
           }
         }
-        if (ANY && hit_any) done = true;
       }
     }
     if constexpr (kCoop) {
@@ -785,7 +799,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
         }
         if (COUNT) ntest += j;
         const unsigned long long mykey =
-            ((unsigned long long)order_key(best_t) << 32) | (uint32_t)best_id;
+            ANY ? 1ull : ((unsigned long long)order_key(best_t) << 32) | (uint32_t)best_id;
         key[lane] = mykey;
         __syncwarp();
         const int nitems = total < 32 ? total : 32;
@@ -872,8 +886,8 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
           if constexpr (W == 8) {
             const uint32_t hk = e.y & 0xffu;
             const uint32_t k = __ffs(hk) - 1;
-            const uint32_t slot =
-                k ^ (kRayShared ? __float_as_uint(s_ray[3 * threadIdx.x + 2].w) : octm);
+            uint32_t slot = k;
+            if (kOctants) slot ^= kRayShared ? __float_as_uint(s_ray[3 * threadIdx.x + 2].w) : octm;
             const uint32_t imask = (e.y >> 8) & 0xffu;
             node = e.x + __popc(imask & ((1u << slot) - 1u));
             const uint32_t rest = hk & (hk - 1u);
@@ -1292,9 +1306,11 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
   // its copies, keeps it whatever the order: leaner, it ran faster but slowed
   // the concurrent copies more (the whole call 4 % slower).
   const bool ord = !ANY && order != nullptr;
-  auto k = lane ? wbvh_trace<W, CLAMP, ANY, COUNT, false, true, true>
-                : (ord ? wbvh_trace<W, CLAMP, ANY, COUNT, false, false, true>
-                       : wbvh_trace<W, CLAMP, ANY, COUNT>);
+  auto k = wbvh_trace<W, CLAMP, ANY, COUNT>;
+  if constexpr (!ANY) {
+    if (lane) k = wbvh_trace<W, CLAMP, false, COUNT, false, true, true>;
+    else if (ord) k = wbvh_trace<W, CLAMP, false, COUNT, false, false, true>;
+  }
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
