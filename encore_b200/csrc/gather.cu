@@ -10,13 +10,24 @@
 // distance to the query, formed with the photon test's own operations on the
 // box's clamped coordinates; rounding is monotone, so that distance never
 // exceeds the squared distance of a photon inside the box and pruning drops
-// nothing the photon test would accept.  The k best candidates are kept in a
-// warp-distributed bounded max-heap: S = ceil(k/32) register slots per lane,
-// slot i on lane i % 32; the maximum and its slot are found with two warp max
-// reductions (redux.sync), and an accepted candidate replaces it.  The search
-// radius is max_dist^2 until k photons are held and the heap maximum
-// afterwards, as in PhotonMap::GetNearestNPhotons (PhotonMap.cpp:224-297), so
-// the result is the exact k-nearest set.
+// nothing the photon test would accept.  Accepted photons are appended to a
+// buffer in shared memory; when a step leaves more than `full` of them, the k
+// nearest are kept (keep_nearest) and their largest distance becomes the search
+// radius; before that it is max_dist^2.  The radius never falls below the k-th
+// distance of the photons seen, so at the end the k nearest of the buffer are the
+// exact k-nearest set, as in PhotonMap::GetNearestNPhotons
+// (PhotonMap.cpp:224-297).
+//
+// What bounds it is instruction issue, not memory (L2 holds what it reads).  A
+// bounded max-heap across the warp's registers, whose maximum every accepted
+// photon replaced with two warp reductions, took 911 us for 300,007 queries of
+// k = 50 in a room of 400,000 photons, 1,346 us for 100,007 of k = 256, and 7.6 ms
+// for 1M of k = 50 that find 600 photons each; the buffer takes 577, 621 us and
+// 3.4 ms, and one query at a time per warp where there are few 18 instead of 43
+// us for 1,007.  `full` = k + max(16, 3k/4): more photons per selection against
+// a radius that shrinks later.  k + 0 / 8 / 16 / 32 / 64 for those: 642 / 611 / 599 /
+// 573 / 572, 792 / 731 / 699 / 621 / 621 us, 4.0 / 3.8 / 3.5 / 3.4 / 3.2 ms; for k = 8:
+// 338 / 334 / 325 / 343 / 349 us.
 //
 // Acceptance is the reference's: FP32 dist^2 = (x*x + y*y) + z*z with separate
 // roundings, dist^2 < r^2, and the stored surface normal equal to the query
@@ -27,6 +38,8 @@
 // (Common.h:36); FP32 accumulation.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "../../include/encore_b200.h"
 #include "photon.h"
 
@@ -35,11 +48,8 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarpsPerBlock = 8;
-// Each inner node pushes at most 32 children and the walk is depth first, so
-// 32 entries per level suffice.
-constexpr int kStack = 32 * kPhotonMaxLevels;
 constexpr unsigned kMaxSteps = 1u << 24;
-// Queries a warp takes from the queue at a time.
+// Queries a warp takes from the queue at a time, at most.
 constexpr unsigned kQueryChunk = 4;
 
 struct GatherParams {
@@ -62,7 +72,9 @@ struct GatherParams {
   uint32_t* counter;  // this launch's query-queue head, zeroed before it
   uint32_t* visits;   // COUNT: 4 words per query (see gather_kernel)
   unsigned nq;
+  unsigned chunk;  // queries a warp takes from the queue at a time; 0: warp w takes query w
   int k;
+  int full;        // candidates a step may leave before the k nearest are kept
   float r2max;
   int ignore_normal;
   int caustic;
@@ -72,51 +84,98 @@ __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); 
 __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
 
-// Stack entries.  An inner-node entry is level << 28 | item (level 1..7);
-// a leaf entry is kLeafEntry | first photon, with the leaf's photon count
-// kept beside it, so a leaf step reads its photons without first loading
-// its range.
+// Stack entries: (item, squared distance of its box).  An inner-node item is
+// level << 28 | index (level 1..7); a leaf item is kLeafEntry | first photon, with
+// the leaf's photon count (at most 32) in the low 6 bits of the distance, so a
+// leaf step reads its photons without first loading its range.  Those bits only
+// lower the distance, by less than 2^-17 of it: a box is then visited that its own
+// distance would just have pruned, and its photons are tested one by one.
 constexpr uint32_t kLeafEntry = 0x80000000u;
+constexpr uint32_t kCountBits = 63u;
 
-// Position of the r-th set bit of m (r counted from 0, r < popc(m)), by
-// halving: keep the low half while it holds more than r set bits.
-__device__ __forceinline__ int nth_set_bit(unsigned m, int r) {
-  int pos = 0;
-#pragma unroll
-  for (int b = 16; b >= 1; b >>= 1) {
-    const int c = __popc(m & ((1u << b) - 1u));
-    if (r >= c) {
-      r -= c;
-      m >>= b;
-      pos += b;
-    }
-  }
-  return pos;
-}
-
-// Max over the slots marked valid (slot index s*32 + lane < limit) and its
-// slot index, the highest slot among equal maxima; -INF / -1 if none.  The
-// held values are squared distances, non-negative floats whose bit patterns
-// order as unsigned integers, so two warp max reductions (redux.sync) find
-// the value and then its slot.
+// The smallest of a warp's candidates: keeps, of the `count` entries of buf
+// (squared distance, photon; count <= 32 S), the k nearest, in their order, and
+// returns the k-th distance.  A threshold with exactly k entries below it is
+// searched between 0 and the largest: on a surface the number of photons within
+// a distance grows with its square, so interpolating the counts finds one in a
+// few steps; after kGuesses of them the interval is halved, and entries of equal
+// distance at its end are kept in order.  Squared distances are non-negative, so
+// their bit patterns order as unsigned integers.
+constexpr int kGuesses = 8;
 template <int S>
-__device__ __forceinline__ void warp_max(const float (&dd)[S], int lane, int limit, float& v,
-                                         int& loc) {
-  uint32_t lv = 0;
-  int ls = -1;
+__device__ __forceinline__ float keep_nearest(uint2* buf, int count, int k, int lane, unsigned lt) {
+  uint2 e[S];
+  uint32_t top = 0;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    const int slot = s * 32 + lane;
-    const uint32_t u = __float_as_uint(dd[s]);
-    if (slot < limit && (ls < 0 || u >= lv)) {
-      lv = u;
-      ls = slot;
-    }
+    e[s] = s * 32 + lane < count ? buf[s * 32 + lane] : make_uint2(~0u, 0u);
+    if (s * 32 + lane < count) top = max(top, e[s].x);
   }
-  const uint32_t mv = __reduce_max_sync(kFull, ls >= 0 ? lv : 0u);
-  const uint32_t l1 = __reduce_max_sync(kFull, (ls >= 0 && lv == mv) ? (uint32_t)(ls + 1) : 0u);
-  loc = (int)l1 - 1;
-  v = l1 == 0 ? -INFINITY : __uint_as_float(mv);
+  uint32_t lo = 0, hi = __reduce_max_sync(kFull, top) + 1;  // keys lie in [lo, hi)
+  int clo = 0, chi = count;                                 // entries below lo and hi
+  int ties = 0;                                             // of value lo that are kept
+  for (int i = 0;; ++i) {
+    if (hi - lo == 1) {
+      ties = k - clo;
+      break;
+    }
+    uint32_t t = lo + (hi - lo) / 2;
+    if (i < kGuesses) {
+      const float flo = __uint_as_float(lo), fhi = __uint_as_float(hi - 1);
+      const float g = flo + (fhi - flo) * ((float)(k - clo) + 0.5f) / (float)(chi - clo);
+      t = min(max(__float_as_uint(g), lo + 1), hi - 1);
+    }
+    int c = 0;
+#pragma unroll
+    for (int s = 0; s < S; ++s) c += __popc(__ballot_sync(kFull, e[s].x < t));
+    if (c == k) {
+      lo = t;
+      break;
+    }
+    if (c < k) lo = t, clo = c;
+    else hi = t, chi = c;
+  }
+  // entries below lo, and the first `ties` of value lo
+  int at = 0;
+  uint32_t far = 0;
+  __syncwarp();
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    bool keep = e[s].x < lo;
+    if (ties > 0) {
+      const unsigned eq = __ballot_sync(kFull, e[s].x == lo);
+      keep = keep || (e[s].x == lo && __popc(eq & lt) < ties);
+      ties -= min(ties, __popc(eq));
+    }
+    const unsigned m = __ballot_sync(kFull, keep);
+    if (keep) {
+      buf[at + __popc(m & lt)] = e[s];
+      far = max(far, e[s].x);
+    }
+    at += __popc(m);
+  }
+  __syncwarp();
+  return __uint_as_float(__reduce_max_sync(kFull, far));
+}
+
+// Bitonic sort of the warp's `count` entries by (first, second) word; n: the
+// power of two >= count, the entries between them set to the largest value.
+__device__ __forceinline__ void sort_entries(uint2* buf, int count, int n, int lane) {
+  for (int i = count + lane; i < n; i += 32) buf[i] = make_uint2(~0u, ~0u);
+  __syncwarp();
+  for (int size = 2; size <= n; size <<= 1)
+    for (int gap = size >> 1; gap > 0; gap >>= 1) {
+      for (int j = lane; j < n / 2; j += 32) {
+        const int i = 2 * j - (j & (gap - 1));
+        const uint2 a = buf[i], b = buf[i + gap];
+        const bool less = b.x < a.x || (b.x == a.x && b.y < a.y);
+        if (less == ((i & size) == 0)) {
+          buf[i] = b;
+          buf[i + gap] = a;
+        }
+      }
+      __syncwarp();
+    }
 }
 
 // COUNT: also records per query the work behind the roofline's bytes:
@@ -125,54 +184,46 @@ __device__ __forceinline__ void warp_max(const float (&dd)[S], int lane, int lim
 // photons found (their 16-byte power is read by the estimate).
 template <int S, bool NEAREST, bool COUNT = false>
 __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
-  // stack entries, their squared distances, and a leaf entry's photon count
-  __shared__ uint32_t s_item[kWarpsPerBlock][kStack];
-  __shared__ float s_pd[kWarpsPerBlock][kStack];
-  __shared__ uint8_t s_cnt[kWarpsPerBlock][kStack];
+  constexpr int kCap = 32 * S;  // candidates a warp holds: k <= kCap - 32
+  // per warp: candidates; stack entries, their squared distances, and a leaf
+  // entry's photon count
+  __shared__ uint2 s_buf[kWarpsPerBlock][kCap];
+  extern __shared__ uint2 s_dyn[];
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int k = P.k;
-  // Each warp takes kQueryChunk queries at a time from the launch's queue
-  // head, so every warp stays busy until the queue is empty (a fixed share
-  // per warp left a fifth of the warp slots idle at the end).  The head
-  // overshoots nq by at most kQueryChunk per warp: nq < 2^31 keeps it below
-  // 2^32.
+  const int depth = 32 * P.nlevels;  // stack entries of a warp
+  uint2* stk = s_dyn + wib * depth;
+  uint2* buf = s_buf[wib];
+  // Each warp takes P.chunk queries at a time from the launch's queue head, so
+  // every warp stays busy until the queue is empty (a fixed share per warp left
+  // a fifth of the warp slots idle at the end).  The head overshoots nq by at
+  // most a chunk per warp: nq < 2^31 keeps it below 2^32.
   unsigned q = 0, qend = 0;
   for (;;) {
     if (q == qend) {
-      unsigned b = 0;
-      if (lane == 0) b = atomicAdd(P.counter, kQueryChunk);
-      b = __shfl_sync(kFull, b, 0);
+      unsigned b = P.nq;
+      if (P.chunk) {
+        if (lane == 0) b = atomicAdd(P.counter, P.chunk);
+        b = __shfl_sync(kFull, b, 0);
+      } else if (qend == 0) {
+        b = blockIdx.x * kWarpsPerBlock + wib;
+      }
       if (b >= P.nq) break;
       q = b;
-      qend = min(b + kQueryChunk, P.nq);
+      qend = min(b + max(P.chunk, 1u), P.nq);
     }
     const float qx = __ldg(P.qpos + 3 * (size_t)q), qy = __ldg(P.qpos + 3 * (size_t)q + 1),
                 qz = __ldg(P.qpos + 3 * (size_t)q + 2);
     const float nx = __ldg(P.qnrm + 3 * (size_t)q), ny = __ldg(P.qnrm + 3 * (size_t)q + 1),
                 nz = __ldg(P.qnrm + 3 * (size_t)q + 2);
-    float dd[S];
-    int ds[S];
-    int dorig[S];
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      dd[s] = INFINITY;
-      ds[s] = 0;
-      dorig[s] = -1;
-    }
     int count = 0;
-    float worst = INFINITY;
-    int worst_loc = -1;
     float r2 = P.r2max;
     // the root: the top level's items are its children
     int sp = 0;
     if (k > 0) {
-      if (lane == 0) {
-        s_item[wib][0] = (uint32_t)P.nlevels << 28;
-        s_pd[wib][0] = 0.f;
-        s_cnt[wib][0] = 0;
-      }
+      if (lane == 0) stk[0] = make_uint2((uint32_t)P.nlevels << 28, 0u);
       sp = 1;
     }
     __syncwarp();
@@ -184,10 +235,9 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
         break;
       }
       --sp;
-      const float pd = s_pd[wib][sp];
-      const uint32_t e = s_item[wib][sp];
-      const int c0 = s_cnt[wib][sp];
-      if (!(pd < r2)) {  // nothing in it can be accepted any more
+      const uint2 top = stk[sp];
+      const uint32_t e = top.x;
+      if (!(__uint_as_float(top.y & ~kCountBits) < r2)) {  // nothing in it can be accepted
         __syncwarp();
         continue;
       }
@@ -214,7 +264,7 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
         const unsigned m = __ballot_sync(kFull, pass);
         if (COUNT) n_box += __popc(__ballot_sync(kFull, child < P.lvl_count[cl]));
         const int n = __popc(m);
-        if (sp + n > kStack) {
+        if (sp + n > depth) {
           if (lane == 0) atomicOr(P.status, 2u);
           break;
         }
@@ -238,9 +288,7 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
             item = kLeafEntry | rng.x;
             cnt = rng.y - rng.x;
           }
-          s_item[wib][at] = item;
-          s_pd[wib][at] = cd;
-          s_cnt[wib][at] = (uint8_t)cnt;
+          stk[at] = make_uint2(item, (__float_as_uint(cd) & ~kCountBits) | cnt);
         }
         sp += n;
         __syncwarp();
@@ -248,13 +296,15 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
       }
       // leaf: lane j tests photon j of the leaf; when the entry below is a
       // leaf too and both fit in the warp, lanes c0.. test its photons
+      const int c0 = (int)(top.y & kCountBits);
       uint32_t b1 = 0;
       int c1 = 0;
       if (sp > 0) {
-        const uint32_t e1 = s_item[wib][sp - 1];
-        const int n1 = s_cnt[wib][sp - 1];
-        if ((e1 & kLeafEntry) && c0 + n1 <= 32 && s_pd[wib][sp - 1] < r2) {
-          b1 = e1 & ~kLeafEntry;
+        const uint2 next = stk[sp - 1];
+        const int n1 = (int)(next.y & kCountBits);
+        if ((next.x & kLeafEntry) && c0 + n1 <= 32 &&
+            __uint_as_float(next.y & ~kCountBits) < r2) {
+          b1 = next.x & ~kLeafEntry;
           c1 = n1;
           --sp;
         }
@@ -264,7 +314,6 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
                                       : b1 + (unsigned)(lane - c0);
       bool acc = false;
       float d2 = 0.f;
-      int orig = -1;
       if (COUNT) {
         n_pos += (uint32_t)(c0 + c1);
       }
@@ -272,7 +321,6 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
         const float4 p = __ldg(P.pos4 + pidx);
         const float x = fs(qx, p.x), y = fs(qy, p.y), z = fs(qz, p.z);
         d2 = fa(fa(fm(x, x), fm(y, y)), fm(z, z));
-        orig = __float_as_int(p.w);
         acc = d2 < r2;
         if (acc && !P.ignore_normal) {
           const float4 pn = __ldg(P.nrm4 + pidx);
@@ -281,102 +329,51 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
       }
       if (COUNT && !P.ignore_normal)
         n_nrm += __popc(__ballot_sync(kFull, lane < c0 + c1 && d2 < r2));
-      unsigned m = __ballot_sync(kFull, acc);
-      if (m && count < k) {
-        // fill free heap slots in one step: the accepted candidate of rank r
-        // (r-th set bit of m) goes to slot count + r, which lives on lane
-        // (count + r) % 32, register (count + r) / 32
-        const int na = __popc(m);
-        const int nfill = min(na, k - count);
-        const int r = (lane - count) & 31;
-        const bool take = r < nfill;
-        const int src = nth_set_bit(m, take ? r : 0);
-        const float cd = __shfl_sync(kFull, d2, src);
-        const int co = __shfl_sync(kFull, orig, src);
-        const int cs = __shfl_sync(kFull, (int)pidx, src);
-        const int slot = count + r;
-        if (take) {
-#pragma unroll
-          for (int s = 0; s < S; ++s)
-            if (s == (slot >> 5)) {
-              dd[s] = cd;
-              ds[s] = cs;
-              dorig[s] = co;
-            }
-        }
-        // the first nfill set bits are done
-        if (nfill == na) {
-          m = 0;
-        } else {
-          for (int i = 0; i < nfill; ++i) m &= m - 1;
-        }
-        count += nfill;
-        if (count == k) {
-          warp_max<S>(dd, lane, k, worst, worst_loc);
-          r2 = worst;
-        }
+      const unsigned m = __ballot_sync(kFull, acc);
+      if (acc) buf[count + __popc(m & lt)] = make_uint2(__float_as_uint(d2), pidx);
+      count += __popc(m);
+      __syncwarp();
+      if (count > P.full) {
+        r2 = keep_nearest<S>(buf, count, k, lane, lt);
+        count = k;
       }
-      // the heap is full (a fill step leaves candidates only then): each
-      // closer candidate replaces the maximum
-      while (m) {
-        const int j = __ffs(m) - 1;
-        m &= m - 1;
-        const float cd = __shfl_sync(kFull, d2, j);
-        const int co = __shfl_sync(kFull, orig, j);
-        const int cs = __shfl_sync(kFull, (int)pidx, j);
-        if (cd < worst) {
-#pragma unroll
-          for (int s = 0; s < S; ++s)
-            if (lane == (worst_loc & 31) && s == (worst_loc >> 5)) {
-              dd[s] = cd;
-              ds[s] = cs;
-              dorig[s] = co;
-            }
-          warp_max<S>(dd, lane, k, worst, worst_loc);
-          r2 = worst;
-        }
-      }
+    }
+    if (count > k) {
+      keep_nearest<S>(buf, count, k, lane, lt);
+      count = k;
     }
 
     if (NEAREST) {
-      // rank = number of held entries ordered before this one (dist^2, index)
-#pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int slot = s * 32 + lane;
-        int rank = 0;
-#pragma unroll
-        for (int s2 = 0; s2 < S; ++s2)
-          for (int l = 0; l < 32; ++l) {
-            const float od = __shfl_sync(kFull, dd[s2], l);
-            const int oo = __shfl_sync(kFull, dorig[s2], l);
-            const int oslot = s2 * 32 + l;
-            if (oslot < count && (od < dd[s] || (od == dd[s] && oo < dorig[s]))) ++rank;
-          }
-        if (slot < count) {
-          P.idx[(size_t)q * k + rank] = dorig[s];
-          P.d2[(size_t)q * k + rank] = dd[s];
-        }
-      }
-      for (int p = count + lane; p < k; p += 32) {
-        P.idx[(size_t)q * k + p] = -1;
-        P.d2[(size_t)q * k + p] = 0.f;
+      // by distance, then by the photon's index
+      for (int i = lane; i < count; i += 32)
+        buf[i].y = (uint32_t)__float_as_int(__ldg(&P.pos4[buf[i].y].w));
+      int n = 2;
+      while (n < count) n <<= 1;
+      sort_entries(buf, count, n, lane);
+      for (int p = lane; p < k; p += 32) {
+        const uint2 c = p < count ? buf[p] : make_uint2(0u, ~0u);
+        P.idx[(size_t)q * k + p] = (int32_t)c.y;
+        P.d2[(size_t)q * k + p] = __uint_as_float(c.x);
       }
       if (lane == 0) P.count[q] = count;
+      __syncwarp();
     } else {
       float R = 0.f, G = 0.f, B = 0.f;
       if (count > 0) {
-        float r;
-        int loc;
-        warp_max<S>(dd, lane, count, r, loc);
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-          if (s * 32 + lane < count) {
-            const float w = P.caustic ? __fdiv_rn(fs(r, dd[s]), dd[s]) : 1.0f;
-            const float4 pw = __ldg(P.pow4 + ds[s]);
-            R = fa(R, fm(pw.x, w));
-            G = fa(G, fm(pw.y, w));
-            B = fa(B, fm(pw.z, w));
-          }
+        float r = 0.f;
+        if (P.caustic) {
+          uint32_t far = 0;
+          for (int i = lane; i < count; i += 32) far = max(far, buf[i].x);
+          r = __uint_as_float(__reduce_max_sync(kFull, far));
+        }
+        for (int i = lane; i < count; i += 32) {
+          const uint2 c = buf[i];
+          const float d = __uint_as_float(c.x);
+          const float w = P.caustic ? __fdiv_rn(fs(r, d), d) : 1.0f;
+          const float4 pw = __ldg(P.pow4 + c.y);
+          R = fa(R, fm(pw.x, w));
+          G = fa(G, fm(pw.y, w));
+          B = fa(B, fm(pw.z, w));
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -396,6 +393,7 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
         P.rgb[3 * (size_t)q + 1] = G;
         P.rgb[3 * (size_t)q + 2] = B;
       }
+      __syncwarp();
     }
     if (COUNT && lane == 0) {
       P.visits[4 * (size_t)q] = n_box;
@@ -440,25 +438,35 @@ int launch_gather(const DevPhotonMap& m, const float* qpos, const float* qnrm, s
   p.r2max = max_dist * max_dist;  // maxDistance*maxDistance in FP32 (PhotonMap.cpp:89)
   p.ignore_normal = (flags & ENC_GATHER_IGNORE_NORMAL) ? 1 : 0;
   p.caustic = m.caustic;
-  const int S = k <= 32 ? 1 : (k <= 64 ? 2 : (k <= 128 ? 4 : 8));
-  void (*kern)(GatherParams) = S == 1   ? gather_kernel<1, NEAREST, COUNT>
-                               : S == 2 ? gather_kernel<2, NEAREST, COUNT>
-                               : S == 4 ? gather_kernel<4, NEAREST, COUNT>
-                                        : gather_kernel<8, NEAREST, COUNT>;
+  int S = 0;
+  void (*kern)(GatherParams) = nullptr;
+  if (k <= 16) S = 2, kern = gather_kernel<2, NEAREST, COUNT>;
+  else if (k <= 32) S = 3, kern = gather_kernel<3, NEAREST, COUNT>;
+  else if (k <= 64) S = 4, kern = gather_kernel<4, NEAREST, COUNT>;
+  else if (k <= 128) S = 6, kern = gather_kernel<6, NEAREST, COUNT>;
+  else S = 10, kern = gather_kernel<10, NEAREST, COUNT>;
+  p.full = std::min(32 * S - 32, k + std::max(16, 3 * k / 4));
+  const size_t smem = (size_t)kWarpsPerBlock * 32 * m.nlevels * sizeof(uint2);
   // One resident wave of persistent warps (the register count allows 5
   // blocks of 256 threads per SM): a larger grid would only queue blocks
   // that find the query queue empty.
   int sms = 148, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device);
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
-  if (e != cudaSuccess) return (int)e;
-  e = cudaMemsetAsync(p.counter, 0, sizeof(uint32_t), s);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
   if (e != cudaSuccess) return (int)e;
   if (per_sm < 1) per_sm = 1;
   const unsigned need = (unsigned)((nq + kWarpsPerBlock - 1) / kWarpsPerBlock);
   unsigned grid = (unsigned)sms * (unsigned)per_sm;
-  if (grid > need) grid = need;
-  kern<<<grid, 256, 0, s>>>(p);
+  const size_t warps = (size_t)grid * kWarpsPerBlock;
+  if (nq <= warps) {
+    p.chunk = 0;  // no more queries than warps: no queue
+    grid = need;
+  } else {
+    p.chunk = (unsigned)std::max<size_t>(1, std::min<size_t>(kQueryChunk, nq / (4 * warps)));
+    e = cudaMemsetAsync(p.counter, 0, sizeof(uint32_t), s);
+    if (e != cudaSuccess) return (int)e;
+  }
+  kern<<<grid, 256, smem, s>>>(p);
   return (int)cudaGetLastError();
 }
 
