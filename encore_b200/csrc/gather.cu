@@ -269,8 +269,8 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
           break;
         }
         // Nearest child on top: the passing children are pushed farthest
-        // first, so the walk visits them nearest first, the heap fills with
-        // nearer photons and its maximum (the search radius once full)
+        // first, so the walk visits them nearest first, the buffer fills with
+        // nearer photons and the search radius, once k are kept,
         // shrinks sooner.  A child's place = the passing children farther
         // than it (equal distances: the higher lane counts as farther).
         int farther = 0;
