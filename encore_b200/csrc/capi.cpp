@@ -222,6 +222,7 @@ Launch resolve_launch(const enc_launch_opts* o, int kind, int width) {
   if (o) {
     if (o->block_threads > 0) L.block = o->block_threads;
     if (o->blocks_per_sm > 0) L.blocks_per_sm = o->blocks_per_sm;
+    L.fixed_shape = o->block_threads > 0 || o->blocks_per_sm > 0;
     if (o->chunk > 0) {
       L.chunk = o->chunk;
       L.fixed_chunk = true;

@@ -196,6 +196,7 @@ struct Launch {
   int blocks_per_sm = 4;
   int chunk = 32;
   bool fixed_chunk = false;  // the caller chose `chunk`
+  bool fixed_shape = false;  // the caller chose the block or the blocks per SM
   int stack = 32;
   // Closest hit with one triangle loop per lane instead of the warp-wide
   // triangle rounds: the host-buffer pipeline uses it (see host_form).

@@ -159,6 +159,22 @@ __device__ __forceinline__ float u8f(uint32_t q) {
   return __uint_as_float(0x4B000000u | q) - 8388608.0f;
 }
 
+// Box tests use a reciprocal with |d| floored at 1e-20 so that a zero
+// direction component (the reference's Normalize clamps small ones to
+// exactly 0) gives finite slab distances instead of 0 * inf = NaN,
+// which would leave that axis unconstrained.  The triangle predicate
+// keeps the exact direction.
+// The hardware reciprocal (rcp.approx, within 1 ulp) is enough here:
+// an error of an ulp scales one axis's slab distances by 1 +- 2^-23,
+// far inside the 1e-5 padding that keeps every accepted hit point off
+// its box's faces, and it saves an IEEE division per axis each time a
+// lane takes a new ray (measured +2.4 % closest, +3 % any hit).
+__device__ __forceinline__ float slab_rcp(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d)));
+  return r;
+}
+
 template <int W>
 struct NodeWords {
   static constexpr int N = WNodeLayout<W>::kBytes / 16;
@@ -477,24 +493,9 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
         ox = r0.x; oy = r0.y; oz = r0.z; tmin = r0.w;
         dx = r1.x; dy = r1.y; dz = r1.z; tmax = r1.w;
 
-        // Box tests use a reciprocal with |d| floored at 1e-20 so that a zero
-        // direction component (the reference's Normalize clamps small ones to
-        // exactly 0) gives finite slab distances instead of 0 * inf = NaN,
-        // which would leave that axis unconstrained.  The triangle predicate
-        // keeps the exact direction.
-        // The hardware reciprocal (rcp.approx, within 1 ulp) is enough here:
-        // an error of an ulp scales one axis's slab distances by 1 +- 2^-23,
-        // far inside the 1e-5 padding that keeps every accepted hit point off
-        // its box's faces, and it saves an IEEE division per axis each time a
-        // lane takes a new ray (measured +2.4 % closest, +3 % any hit).
-        auto rcp = [](float x) {
-          float r;
-          asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-          return r;
-        };
-        ix = rcp(fabsf(dx) > 1e-20f ? dx : copysignf(1e-20f, dx));
-        iy = rcp(fabsf(dy) > 1e-20f ? dy : copysignf(1e-20f, dy));
-        iz = rcp(fabsf(dz) > 1e-20f ? dz : copysignf(1e-20f, dz));
+        ix = slab_rcp(dx);
+        iy = slab_rcp(dy);
+        iz = slab_rcp(dz);
         octm = (dx < 0.f ? 1u : 0u) | (dy < 0.f ? 2u : 0u) | (dz < 0.f ? 4u : 0u);
         if (kCoop) {
           s_ray[3 * threadIdx.x] = r0;
@@ -944,6 +945,208 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
 }
 
 // ---------------------------------------------------------------------------
+// Few rays: eight lanes walk one ray, one child box each.
+//
+// A batch that leaves most of the GPU idle takes as long as its longest ray, and
+// a step of wbvh_trace costs a lone warp about 1 us: the node's load, eight slab
+// tests, the triangles' load and the triangle round, one after another.  Here
+// lane c of a ray's eight tests child c, then the leaf triangles that the step
+// reached, eight at a time, while the next node is already on its way (which node
+// that is depends on neither).  The stack and the walk are wbvh_trace's for
+// width 8, child order, culling and the choice among candidates included, so the
+// hits are the same bits.  777 / 5,000 eye and bounce rays in 10,000 triangles: 49
+// / 66 us with a share of rays per warp, 33 / 43 us here (39 / 49 with the next
+// node fetched after the triangles); 777 shadow rays 58 -> 41.  Prefetching the
+// other children hit to L1 made 5,000 rays 2 us slower.
+
+// Position of the r-th set bit of m (r counted from 0, r < popc(m)), by
+// halving: keep the low half while it holds more than r set bits.
+__device__ __forceinline__ int nth_set_bit(unsigned m, int r) {
+  int pos = 0;
+#pragma unroll
+  for (int b = 16; b >= 1; b >>= 1) {
+    const int c = __popc(m & ((1u << b) - 1u));
+    if (r >= c) {
+      r -= c;
+      m >>= b;
+      pos += b;
+    }
+  }
+  return pos;
+}
+
+template <bool CLAMP, bool ANY>
+__global__ void __launch_bounds__(128) wbvh_few(TraceParams P) {
+  using L = WNodeLayout<8>;
+  extern __shared__ uint2 s_stack[];
+  const unsigned lane = threadIdx.x & 31u, grp = lane >> 3, c = lane & 7u;
+  uint2* stk = s_stack + (size_t)(threadIdx.x >> 3) * P.stack_depth;
+  const unsigned q = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * P.share + grp;
+  bool live = grp < P.share && q < P.nrays;
+  unsigned ray = q;
+  if (live && P.order) {
+    ray = __ldg(P.order + q);
+    if (ray >= P.nrays) {  // an order entry outside the batch: skipped and reported
+      if (c == 0) atomicOr(P.status, kStatusBounds);
+      live = false;
+    }
+  }
+  float ox = 0, oy = 0, oz = 0, dx = 0, dy = 0, dz = 0, tmin = 0, tmax = 0;
+  if (live) {
+    const float4 r0 = __ldg(P.rays + 2 * (size_t)ray), r1 = __ldg(P.rays + 2 * (size_t)ray + 1);
+    ox = r0.x; oy = r0.y; oz = r0.z; tmin = r0.w;
+    dx = r1.x; dy = r1.y; dz = r1.z; tmax = r1.w;
+  }
+  const float ix = slab_rcp(dx), iy = slab_rcp(dy), iz = slab_rcp(dz);
+  const uint32_t octm = (dx < 0.f ? 1u : 0u) | (dy < 0.f ? 2u : 0u) | (dz < 0.f ? 4u : 0u);
+  // the byte of child c in the near and far plane array of each axis
+  const unsigned nx = L::kQOff + (octm & 1u ? 24u : 0u) + c, fx = L::kQOff + (octm & 1u ? 0u : 24u) + c;
+  const unsigned ny = L::kQOff + (octm & 2u ? 32u : 8u) + c, fy = L::kQOff + (octm & 2u ? 8u : 32u) + c;
+  const unsigned nz = L::kQOff + (octm & 4u ? 40u : 16u) + c, fz = L::kQOff + (octm & 4u ? 16u : 40u) + c;
+  float best_t = tmax, bu = 0.f, bv = 0.f;
+  int best_id = -1;
+  bool hit_any = false, lost = false;  // lost: stopped at a bound, reported as a miss
+  int sp = 0;
+  unsigned steps = 0;
+  uint32_t node = live ? 0u : kNoItem;
+  // the node to visit: its header and child c's planes
+  uint4 h0 = make_uint4(0, 0, 0, 0), h1 = h0;
+  uint32_t pnx = 0, pfx = 0, pny = 0, pfy = 0, pnz = 0, pfz = 0;
+  auto fetch = [&]() {
+    if (node == kNoItem) return;
+    if (++steps > kMaxSteps || node >= P.nnodes) {
+      if (c == 0) atomicOr(P.status, steps > kMaxSteps ? kStatusWatchdog : kStatusBounds);
+      lost = true;
+      node = kNoItem;
+      return;
+    }
+    const uint8_t* src = P.nodes + (size_t)node * L::kBytes;
+    h0 = __ldg(reinterpret_cast<const uint4*>(src));
+    h1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+    pnx = __ldg(src + nx), pfx = __ldg(src + fx);
+    pny = __ldg(src + ny), pfy = __ldg(src + fy);
+    pnz = __ldg(src + nz), pfz = __ldg(src + fz);
+  };
+  fetch();
+
+  while (__any_sync(kFull, node != kNoItem)) {
+    const bool on = node != kNoItem;
+    bool hit = false;
+    if (on) {
+      const float sx = __uint_as_float((h0.w & 0xffu) << 23);
+      const float sy = __uint_as_float(((h0.w >> 8) & 0xffu) << 23);
+      const float sz = __uint_as_float(((h0.w >> 16) & 0xffu) << 23);
+      const float bx = (__uint_as_float(h0.x) - ox) * ix, by = (__uint_as_float(h0.y) - oy) * iy,
+                  bz = (__uint_as_float(h0.z) - oz) * iz;
+      const float cx = sx * ix, cy = sy * iy, cz = sz * iz;
+      const float tnx = fmaf(u8f(pnx), cx, bx), tfx = fmaf(u8f(pfx), cx, bx);
+      const float tny = fmaf(u8f(pny), cy, by), tfy = fmaf(u8f(pfy), cy, by);
+      const float tnz = fmaf(u8f(pnz), cz, bz), tfz = fmaf(u8f(pfz), cz, bz);
+      hit = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tmin)) <= fminf(fminf(tfx, tfy), fminf(tfz, best_t));
+    }
+    const uint32_t hm = (__ballot_sync(kFull, hit) >> (8 * grp)) & 0xffu;
+    const uint32_t imask = h0.w >> 24, tri_base = h1.y;
+    // the triangles of the hit leaves: lane c's leaf, then the eight together
+    const uint32_t meta = ((c & 4u ? h1.w : h1.z) >> ((c & 3u) * 8u)) & 0xffu;
+    uint32_t tris = hit && !((imask >> c) & 1u) ? ((1u << (meta >> 5)) - 1u) << (meta & 31u) : 0u;
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) tris |= __shfl_xor_sync(kFull, tris, d);
+    // ---- the next node: the first child hit, else the deferred child pushed
+    //      last.  Neither depends on the triangles (a child is culled when its
+    //      box is tested), so its data is on its way while they are tested.
+    uint32_t x = on ? hm & imask : 0u;
+    if (!ANY) {
+      if (octm & 1u) x = ((x & 0x55u) << 1) | ((x >> 1) & 0x55u);
+      if (octm & 2u) x = ((x & 0x33u) << 2) | ((x >> 2) & 0x33u);
+      if (octm & 4u) x = ((x & 0x0fu) << 4) | ((x >> 4) & 0x0fu);
+    }
+    const bool pop = on && x == 0 && sp > 0;
+    const uint2 e = pop ? stk[sp - 1] : make_uint2(h1.x, x | (imask << 8));
+    __syncwarp();  // all eight have read it
+    if (on) {
+      node = kNoItem;
+      const uint32_t hk = e.y & 0xffu;
+      if (hk) {
+        const uint32_t k = __ffs(hk) - 1, slot = ANY ? k : k ^ octm, rest = hk & (hk - 1u);
+        node = e.x + __popc((e.y >> 8) & ((1u << slot) - 1u));
+        if (pop) --sp;
+        if (rest && sp >= P.stack_depth) {
+          if (c == 0) atomicOr(P.status, kStatusStack);
+          lost = true;
+          node = kNoItem;
+        } else if (rest) {
+          if (c == 0) stk[sp] = make_uint2(e.x, (e.y & ~0xffu) | rest);
+          ++sp;
+        }
+      }
+    }
+    fetch();
+    // ---- triangles, eight at a time ---------------------------------------
+    while (__any_sync(kFull, tris != 0)) {
+      const int n = __popc(tris);
+      unsigned long long key = ~0ull;
+      float u = 0.f, v = 0.f;
+      if ((int)c < n) {
+        const uint32_t ti = tri_base + (uint32_t)nth_set_bit(tris, (int)c);
+        if (ti >= P.ntris) {
+          atomicOr(P.status, kStatusBounds);
+        } else {
+          const float4* tp = P.tris + 3 * (size_t)ti;
+          const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+          float t;
+          if (tri_test<CLAMP>(ta, tb, tc, ox, oy, oz, dx, dy, dz, tmin, t, u, v)) {
+            const int id = __float_as_int(tc.y);
+            if (t < best_t || (!ANY && t == best_t && id < best_id))
+              key = ((unsigned long long)order_key(t) << 32) | (uint32_t)id;
+          }
+        }
+      }
+      if (ANY) {
+        if ((__ballot_sync(kFull, key != ~0ull) >> (8 * grp)) & 0xffu) {
+          hit_any = true;
+          node = kNoItem;
+          tris = 0;
+        }
+      } else {
+        unsigned long long low = key;
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) {
+          const unsigned long long o = __shfl_xor_sync(kFull, low, d);
+          low = o < low ? o : low;
+        }
+        // (two triangles of one ID cannot occur: IDs are a permutation)
+        const uint32_t from = (__ballot_sync(kFull, key == low) >> (8 * grp)) & 0xffu;
+        const int src = (int)(8 * grp) + __ffs(from) - 1;
+        const float wu = __shfl_sync(kFull, u, src), wv = __shfl_sync(kFull, v, src);
+        if (low != ~0ull) {
+          best_t = from_order_key((uint32_t)(low >> 32));
+          best_id = (int)(uint32_t)low;
+          bu = wu;
+          bv = wv;
+        }
+      }
+      if (n <= 8) {
+        tris = 0;
+      } else {
+        for (int i = 0; i < 8; ++i) tris &= tris - 1u;
+      }
+    }
+    __syncwarp();  // the stack entries written above
+  }
+  if (lost) best_id = -1, hit_any = false;
+  if (live && c == 0) {
+    if (ANY) {
+      reinterpret_cast<uint8_t*>(P.out)[ray] = hit_any ? 1 : 0;
+    } else {
+      reinterpret_cast<int4*>(P.out)[ray] =
+          best_id >= 0 ? make_int4(best_id, __float_as_int(best_t), __float_as_int(bu),
+                                   __float_as_int(bv))
+                       : make_int4(-1, 0, 0, 0);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // kd-tree walk in the reference's order (Kdtree.cpp:682-784).
 
 struct KdParams {
@@ -1277,6 +1480,26 @@ unsigned ray_share(const Launch& L, size_t n, int sms, int* grid) {
   return (unsigned)share;
 }
 
+// The largest batch that wbvh_few takes, in warps of four rays per SM (18,944
+// rays on 148 SMs): at 19,000 rays it took 65 us against 79 in 10,000 random
+// triangles, 41 against 61 on a 131,072-triangle field and 70 against 99 for
+// shadow rays, at 38,000 rays 98 against 92, 62 against 70 and 103 against 99.  A
+// caller's choice of chunk, block or blocks per SM is one of wbvh_trace's shape.
+constexpr int kFewWarps = 32;
+bool few_rays(const Launch& L, size_t n, int sms) {
+  return !L.fixed_chunk && !L.fixed_shape && n <= (size_t)sms * kFewWarps * 4;
+}
+template <bool CLAMP, bool ANY>
+int launch_few(TraceParams p, size_t n, int sms, cudaStream_t s) {
+  const size_t warps = (size_t)sms * kSpreadWarps;
+  p.share = (unsigned)std::min<size_t>(4, (n + warps - 1) / warps);  // rays per warp
+  if (n == 0) p.share = 1;  // a warm-up launch: one block that finds no ray
+  const size_t smem = (size_t)16 * p.stack_depth * sizeof(uint2);  // 16 rays per block
+  const unsigned grid = (unsigned)std::max<size_t>(1, (n + 4 * p.share - 1) / (4 * p.share));
+  wbvh_few<CLAMP, ANY><<<grid, 128, smem, s>>>(p);
+  return (int)cudaGetLastError();
+}
+
 template <int W, bool CLAMP, bool ANY, bool COUNT>
 int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t* visits,
              const Launch& L, cudaStream_t s, const uint32_t* order) {
@@ -1298,6 +1521,10 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
   // entries always suffice; 0 selects that bound.
   p.stack_depth = L.stack > 0 ? L.stack : (a.tree_depth > 8 ? a.tree_depth : 8);
   p.chunk = L.chunk;
+  const int sms = device_sm_count(a.device);
+  if constexpr (W == 8 && !COUNT) {
+    if (few_rays(L, n, sms)) return launch_few<CLAMP, ANY>(p, n, sms, s);
+  }
   size_t smem = (size_t)p.stack_depth * L.block * stack_entry_bytes(W);
   const bool lane = !ANY && L.per_lane;
   // Binned (ordered) launches use their own instantiation (closest hit
@@ -1315,7 +1542,6 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  const int sms = device_sm_count(a.device);
   int grid = sms * (L.blocks_per_sm > 0
                         ? L.blocks_per_sm
                         : (ANY ? kBlocksAny : (lane ? kBlocksLane : kBlocksClosest)));
@@ -1430,13 +1656,19 @@ int launch_w_external(const DevAccel& a, const float* rays, size_t n, enc_hit* h
   p.ntris = a.ntris;
   p.stack_depth = L.stack > 0 ? L.stack : (a.tree_depth > 8 ? a.tree_depth : 8);
   p.chunk = L.chunk;
+  const int sms = device_sm_count(a.device);
+  if constexpr (W == 8) {  // the warm-up launch (n = 0) runs both kernels
+    if (few_rays(L, n, sms)) {
+      const int e = launch_few<CLAMP, false>(p, n, sms, s);
+      if (e != 0 || n > 0) return e;
+    }
+  }
   size_t smem = (size_t)p.stack_depth * L.block * stack_entry_bytes(W);
   auto k = wbvh_trace<W, CLAMP, false, false>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  const int sms = device_sm_count(a.device);
   int grid = sms * (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksClosest);
   if (n > 0) p.share = ray_share(L, n, sms, &grid);
   k<<<grid, L.block, smem, s>>>(p);
@@ -1446,6 +1678,7 @@ int launch_w_external(const DevAccel& a, const float* rays, size_t n, enc_hit* h
 }  // namespace
 
 int warm_closest_kernel(const DevAccel& a, uint32_t* counter, uint32_t* status) {
+  // (not fixed_shape: the small-batch kernel is warmed with the other)
   // An empty batch: every warp finds the queue exhausted at once.  The launch
   // loads the kernel's module and sizes the context's local memory for it.
   Launch L = resolve_launch(nullptr, a.kind, a.width);
