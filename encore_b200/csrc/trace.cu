@@ -1176,8 +1176,10 @@ struct KdParams {
 //      the list) below the owner's best is the same item.
 // Lanes whose walk is over take new rays once kKdRefill of them are idle, so
 // the set-up's six divisions run for several lanes at a time.
-// Measured on that batch: 5,190 us one thread per ray, 2,114 us now (1.60 G
-// warp instructions at 25 lanes); kKdLeave 4 / 8 / 12 / 20 / 24: 2,308 / 2,210 /
+// Measured on that batch: 5,190 us one thread per ray, 2,114 us with every leaf
+// in the list (1.60 G warp instructions at 25 lanes), 1,923 with long leaves by
+// themselves (from 24 / 32 / 48 / 96 items: 1,944 / 1,937 / 1,924 / 1,922); with the
+// list, kKdLeave 4 / 8 / 12 / 20 / 24: 2,308 / 2,210 /
 // 2,152 / 2,155 / 2,260; kKdRefill 1 / 4 / 16: within 1 %; 6 / 7 / 9 / 10 blocks
 // per SM: 2,441 / 2,253 / 2,200 / 2,560.  What bounds it now: issue (73 %
 // active) and the latency of its dependent node, item and triangle loads (L2 hit
@@ -1191,14 +1193,16 @@ constexpr unsigned kKdChunk = 32;  // rays a warp takes from the queue at a time
 // memory.
 constexpr int kKdShared = 12;
 constexpr int kKdStack = 64;
-// Items of one leaf listed at a time: bounds the list of 32 leaves.
-constexpr uint32_t kKdLeafItems = 1u << 16;
+// A leaf of so many items or more is tested by itself, with no list and no
+// shared-memory minimum per round: cells at the tree's depth limit hold hundreds
+// (5 % of the field's leaves held 70 % of the tests, 362 items each).
+constexpr uint32_t kKdLong = 64;
 
 template <bool CLAMP, bool ANY>
 __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
   __shared__ uint2 s_stack[kKdShared][128];
-  __shared__ float s_o[3][128], s_d[3][128], s_inv[3][128];
-  __shared__ float2 s_lim[128];              // the ray's tmin and tmax
+  __shared__ float s_o[3][128], s_inv[3][128];  // for the walk: by axis
+  __shared__ float4 s_from[128], s_dir[128];    // for the tests: o, tmin; d, tmax
   __shared__ unsigned long long s_key[128];  // best candidate of the lane's leaf
   __shared__ float4 s_hit[128];              // t, u, v, ID of the ray's closest hit so far
   __shared__ uint8_t s_own[128];             // r-th lane of the warp that has leaf items
@@ -1267,7 +1271,6 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           s_o[i][tid] = o[i];
-          s_d[i][tid] = d[i];
           s_inv[i][tid] = __fdiv_rn(1.f, d[i]);
           if (in) {
             float tin = __fdiv_rn(fs(P.lo[i], o[i]), d[i]);
@@ -1282,7 +1285,8 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
             if (t0 > t1) in = false;
           }
         }
-        s_lim[tid] = make_float2(r0.w, r1.w);
+        s_from[tid] = r0;
+        s_dir[tid] = r1;
         s_hit[tid] = make_float4(INFINITY, 0.f, 0.f, __int_as_float(-1));
         best_t = INFINITY;
         tmin = t0;
@@ -1371,26 +1375,62 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
     }
 
     // ---- the warp tests the items of its lanes' leaves together -----------
+    // Long leaves one by one: all lanes test the same ray, lane l items l, l + 32,
+    // ..., and keep the first nearest of theirs.
+    for (unsigned big = __ballot_sync(kFull, cnt >= kKdLong); big; big &= big - 1u) {
+      const int src = __ffs(big) - 1;
+      const unsigned ot = wbase + (unsigned)src;
+      const uint32_t n = __shfl_sync(kFull, cnt, src);
+      const uint32_t* items = P.items + __shfl_sync(kFull, beg, src);
+      const float4 o = s_from[ot], d = s_dir[ot];
+      float4 near = make_float4(__shfl_sync(kFull, best_t, src), 0.f, 0.f, __int_as_float(-1));
+      uint32_t at = ~0u;
+      for (uint32_t k = lane; k < n; k += 32) {
+        const uint32_t id = __ldg(items + k);
+        if (id >= P.ntris) {
+          atomicOr(P.status, kStatusBounds);
+          continue;
+        }
+        const float4* tp = P.tris + 3 * (size_t)id;
+        float t, u, v;
+        if (tri_test<CLAMP>(__ldg(tp), __ldg(tp + 1), __ldg(tp + 2), o.x, o.y, o.z, d.x, d.y, d.z,
+                            o.w, t, u, v) &&
+            t < near.x) {
+          near = make_float4(t, u, v, __int_as_float((int)id));
+          at = k;
+        }
+      }
+      // the smallest t, then the first in the list (-0 and +0 are one distance)
+      const uint32_t key = at != ~0u ? order_key(near.x == 0.0f ? 0.0f : near.x) : ~0u;
+      const uint32_t low = __reduce_min_sync(kFull, key);
+      const uint32_t first = __reduce_min_sync(kFull, key == low ? at : ~0u);
+      if (first != ~0u && at == first) s_hit[ot] = near;
+      __syncwarp();
+      if ((int)lane == src) {
+        if (first != ~0u) best_t = s_hit[ot].x;
+        cnt = 0;
+        if (!pop()) fin = true;
+      }
+    }
     const unsigned leaves = __ballot_sync(kFull, cnt != 0);
     if (leaves) {
-      const uint32_t take = min(cnt, kKdLeafItems);
-      uint32_t excl = take;  // becomes the lane's first item in the warp's list
+      uint32_t excl = cnt;  // becomes the lane's first item in the warp's list
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const uint32_t v = __shfl_up_sync(kFull, excl, d);
         if ((int)lane >= d) excl += v;
       }
       const uint32_t total = __shfl_sync(kFull, excl, 31);
-      excl -= take;
-      if (take) s_own[wbase + __popc(leaves & lt)] = (uint8_t)lane;
+      excl -= cnt;
+      if (cnt) s_own[wbase + __popc(leaves & lt)] = (uint8_t)lane;
       s_key[tid] = ~0ull;
       __syncwarp();
       for (uint32_t base = 0; base < total; base += 32) {
         // the owner of item base + lane: the last lane whose list starts at
         // or before it
-        const bool starts = take && excl >= base && excl < base + 32;
+        const bool starts = cnt && excl >= base && excl < base + 32;
         const uint32_t first = __reduce_or_sync(kFull, starts ? 1u << (excl - base) : 0u);
-        const unsigned before = __popc(__ballot_sync(kFull, take && excl < base));
+        const unsigned before = __popc(__ballot_sync(kFull, cnt && excl < base));
         const unsigned own = s_own[wbase + before + __popc(first & (lt | (1u << lane))) - 1];
         const uint32_t oexcl = __shfl_sync(kFull, excl, own);
         const uint32_t obeg = __shfl_sync(kFull, beg, own);
@@ -1407,9 +1447,9 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
             atomicOr(P.status, kStatusBounds);
           } else {
             const float4* tp = P.tris + 3 * (size_t)id;
-            if (tri_test<CLAMP>(__ldg(tp), __ldg(tp + 1), __ldg(tp + 2), s_o[0][ot], s_o[1][ot],
-                                s_o[2][ot], s_d[0][ot], s_d[1][ot], s_d[2][ot], s_lim[ot].x, t, u,
-                                v) &&
+            const float4 o = s_from[ot], d = s_dir[ot];
+            if (tri_test<CLAMP>(__ldg(tp), __ldg(tp + 1), __ldg(tp + 2), o.x, o.y, o.z, d.x, d.y,
+                                d.z, o.w, t, u, v) &&
                 t < obest) {
               cand = true;
               // -0 and +0 are one distance: the first of them in the list wins
@@ -1422,11 +1462,10 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
         if (cand && s_key[ot] == key) s_hit[ot] = make_float4(t, u, v, __int_as_float((int)id));
         __syncwarp();
       }
-      if (take) {
+      if (cnt) {
         if (s_key[tid] != ~0ull) best_t = s_hit[tid].x;
-        cnt -= take;
-        beg += take;
-        if (cnt == 0 && !pop()) fin = true;
+        cnt = 0;
+        if (!pop()) fin = true;
       }
     }
 
@@ -1436,7 +1475,7 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
       // beyond the ray's tmax are reported as misses.
       const float4 h = s_hit[tid];
       const int id = lost ? -1 : __float_as_int(h.w);
-      const bool hit = id >= 0 && h.x < s_lim[tid].y;
+      const bool hit = id >= 0 && h.x < s_dir[tid].w;
       if (ANY) {
         reinterpret_cast<uint8_t*>(P.out)[ray] = hit ? 1 : 0;
       } else {

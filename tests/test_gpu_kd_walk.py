@@ -30,11 +30,14 @@ def piled(n, copies, seed):
 
 SCENES = {"soup": lambda: scenes.random_triangles(6000, seed=71, scale=SCALE),
           "piled": lambda: piled(60, 150, seed=72),
+          "one63": lambda: piled(1, 63, seed=75), "one64": lambda: piled(1, 64, seed=75),
+          "one65": lambda: piled(1, 65, seed=75),
           "field": lambda: scenes.heightfield(res=160, seed=73, scale=SCALE)}
 
 
 @pytest.mark.parametrize("name,n", [("soup", 1), ("soup", 33), ("soup", 148 * 16 + 1),
                                     ("soup", 148 * 8 * 4 * 32 + 1), ("piled", 3000),
+                                    ("one63", 900), ("one64", 900), ("one65", 900),
                                     ("field", 40000)])
 @pytest.mark.parametrize("predicate", ["reference", "noclamp"])
 def test_walk_equals_the_oracle(gpu, name, n, predicate):
