@@ -299,7 +299,7 @@ __device__ __forceinline__ void sort_net<4>(float (&k)[4], uint32_t (&v)[4]) {
 #undef ENC_CSWAP
 
 template <int W, bool CLAMP, bool ANY, bool COUNT, bool MULTI = false, bool LANE = false,
-          bool ORD = false>
+          bool ORD = false, bool WAIT = false>
 __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
                                       : LANE ? kBlocksLane
                                              : (MULTI ? kBlocksMulti : kBlocksClosest))
@@ -341,6 +341,19 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   // 371, 16 scenes in one launch 1,157 / 1,143 / 1,134 / 1,143 / 1,160 / 1,211, the
   // shadow rays above 670 / 666 / 663 / 668 / 679 / 703.
   constexpr int kRefill = LANE ? 1 : 4;
+  // With WAIT, lanes that stand at leaves wait for their triangle round until
+  // kWait of them do, while the others walk on: a round costs about as much as
+  // a node visit and listed 10 items of 32.  A lane never walks past a leaf it has
+  // not tested, so its walk is the same.  Once the queue is empty no lane waits,
+  // for the launch then lasts as long as its longest rays.  At 1 / 3 / 4 / 5 / 6 / 8
+  // / 10 / 12 lanes: the heightfield's 4.18M rays 1,155 / 1,138 / 1,116 / 1,099 /
+  // 1,089 / 1,084 / 1,094 / 1,119 us (1,142 without WAIT), 4M eye rays on 10,000
+  // triangles 1,096 / 1,111 / 1,095 / 1,080 / 1,070 / 1,060 / 1,065 / 1,080 (1,083), 16
+  // scenes in one launch 1,136 / 1,147 / 1,135 / 1,124 / 1,115 / 1,105 / 1,108 / 1,131
+  // (1,135).  Any hit gains 6 % where few rays are blocked and loses 2 % where
+  // half are, so it does without.
+  static_assert(!WAIT || kCoop, "the per-lane form has no triangle rounds");
+  constexpr int kWait = 8;
   // the per-lane form keeps the group bound (without it ptxas spills more)
   constexpr bool kBound = kGroupBound || LANE;
   // L2 priorities in the single-scene cooperative closest-hit form only: in
@@ -402,6 +415,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   void* l_out = P.out;
   unsigned l_idx = 0;          // index of the ray in its output array
   unsigned pool_batch = 0;     // MULTI: batch of the current pool
+  uint32_t tmask = 0, tbase = 0;  // untested triangles of the lane's node
   uint32_t* l_status = P.status;  // the status word of the lane's ray (MULTI: its batch's)
 
   while (true) {
@@ -516,8 +530,8 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
 
     bool done = false;
     bool hit_any = false;
-    uint32_t tmask = 0, tbase = 0;  // triangles of the node's hit leaves
-    if (ray >= 0) {
+    if (!WAIT) tmask = 0;
+    if (ray >= 0 && (!WAIT || tmask == 0)) {
       if (++steps > kMaxSteps) {
         atomicOr(l_status, kStatusWatchdog);
         best_id = -1;
@@ -699,6 +713,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
                 atomicOr(l_status, kStatusStack);
                 best_id = -1;
                 done = true;
+                trimask = 0;
               } else {
                 if constexpr (kCompact) {
                   const uint32_t lb16 =
@@ -724,6 +739,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
                 atomicOr(l_status, kStatusStack);
                 best_id = -1;
                 done = true;
+                trimask = 0;
               } else {
                 uint32_t packed = 0;
 #pragma unroll
@@ -776,6 +792,8 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
     // "t < best_t, or equal t and a lower ID", whatever the order.
     {
       unsigned pend = __ballot_sync(kFull, tmask != 0);
+      if (WAIT && !exhausted && __popc(pend) < kWait && pend != __ballot_sync(kFull, ray >= 0))
+        pend = 0;
       const unsigned wib = threadIdx.x >> 5;
       uint32_t* it_tri = s_coop_tri + wib * 32;
       uint32_t* it_own = s_coop_own + wib * 32;
@@ -866,7 +884,7 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
       }
     }
     }
-    if (ray >= 0) {
+    if (ray >= 0 && (!WAIT || tmask == 0)) {
       // ---- pop the next group child that can still matter ----------------
       if (!done && node == kNoItem) {
         while (sp > 0) {
@@ -1528,6 +1546,14 @@ constexpr int kFewWarps = 32;
 bool few_rays(const Launch& L, size_t n, int sms) {
   return !L.fixed_chunk && !L.fixed_shape && n <= (size_t)sms * kFewWarps * 4;
 }
+// Launches long enough for WAIT to pay: six chunks of 32 rays per resident warp
+// (1,022,976 rays).  At 300,000 / 524,288 / 1M / 2M / 4M eye and bounce rays on
+// 10,000 to 100,000 triangles it took 315 / 225 / 342 / 584 / 1,060 us against 305 /
+// 222 / 343 / 592 / 1,083 without.
+bool many_rays(size_t n, int blocks, int threads) {
+  return n >= (size_t)blocks * (size_t)threads * 6;
+}
+
 template <bool CLAMP, bool ANY>
 int launch_few(TraceParams p, size_t n, int sms, cudaStream_t s) {
   const size_t warps = (size_t)sms * kSpreadWarps;
@@ -1576,6 +1602,12 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
   if constexpr (!ANY) {
     if (lane) k = wbvh_trace<W, CLAMP, false, COUNT, false, true, true>;
     else if (ord) k = wbvh_trace<W, CLAMP, false, COUNT, false, false, true>;
+    if constexpr (W == 8 && !COUNT) {
+      const int blocks = sms * (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksClosest);
+      if (!lane && many_rays(n, blocks, L.block))
+        k = ord ? wbvh_trace<W, CLAMP, false, false, false, false, true, true>
+                : wbvh_trace<W, CLAMP, false, false, false, false, false, true>;
+    }
   }
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1781,6 +1813,12 @@ int launch_multi_w(const MultiLaunch& m, const Launch& L, cudaStream_t s) {
   p.batch_status = m.d_batch_status;
   size_t smem = (size_t)p.stack_depth * L.block * stack_entry_bytes(W);
   auto k = wbvh_trace<W, CLAMP, ANY, false, true>;
+  if constexpr (W == 8 && !ANY) {
+    const int blocks = device_sm_count(m.device) *
+                       (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksMulti);
+    if (many_rays(m.total, blocks, L.block))
+      k = wbvh_trace<W, CLAMP, false, false, true, false, false, true>;
+  }
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
