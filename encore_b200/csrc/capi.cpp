@@ -346,6 +346,7 @@ enc_status enc_accel_build(enc_scene scene, const enc_build_opts* opts, int32_t 
       if (e == cudaSuccess) e = upload(&d.d_tri_pos, h.tri_pos.data(), h.tri_pos.size());
       d.node_bytes = h.nodes.size();
       d.tri_bytes = h.tris.size() * sizeof(DevTri);
+      d.tests_per_visit = tests_per_visit(h);
       // keep the tree for refits (not the triangle records: refit rewrites them)
       h.tris.clear();
       h.tris.shrink_to_fit();
@@ -652,6 +653,7 @@ enc_status enc_accel_deserialize(const void* buf, size_t size, int32_t device, e
         hh.lo[i] = h.lo[i];
         hh.hi[i] = h.hi[i];
       }
+      d.tests_per_visit = tests_per_visit(hh);
       uint8_t* dn = nullptr;
       e = upload(&dn, hh.nodes.data(), hh.nodes.size());
       d.d_nodes = dn;
@@ -1629,7 +1631,7 @@ enc_status enc_batch_create(const enc_batch_item* items, uint32_t nitems,
   std::vector<const DevAccel*> uniq;
   std::vector<BatchDesc> batches(nitems);
   std::vector<uint32_t> starts(nitems + 1);
-  uint64_t pos = 0;
+  uint64_t pos = 0, few_tests = 0;
   int depth = 8;
   for (uint32_t i = 0; i < nitems; ++i) {
     const DevAccel* a = accel_device_view(items[i].accel);
@@ -1652,6 +1654,7 @@ enc_status enc_batch_create(const enc_batch_item* items, uint32_t nitems,
     }
     batches[i] = BatchDesc{items[i].d_rays, items[i].d_hits, si, items[i].nrays, (uint32_t)pos, 0};
     starts[i] = (uint32_t)pos;
+    if (a->tests_per_visit < kFewTestsMulti) few_tests += items[i].nrays;
     pos += ((uint64_t)items[i].nrays + L.chunk - 1) / L.chunk * L.chunk;
     if (pos > 0x7fffffffull) {
       set_error("enc_batch_create: more than 2^31 rays in one batch table");
@@ -1682,6 +1685,7 @@ enc_status enc_batch_create(const enc_batch_item* items, uint32_t nitems,
   m.predicate = first->predicate;
   m.device = first->device;
   m.stack_depth = depth;
+  m.wait = 2 * few_tests > pos;
   m.d_counter = b->d_words;
   m.d_status = b->d_words + 1;
   *out = b;

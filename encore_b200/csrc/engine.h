@@ -79,6 +79,7 @@ struct DevAccel {
   uint32_t ntris = 0;
   uint32_t nnodes = 0;
   int tree_depth = 0;  // WBVH levels; the traversal stack needs at most depth - 1 entries
+  float tests_per_visit = 1.f;  // WBVH of width 8: see tests_per_visit()
   // WBVH
   void* d_nodes = nullptr;      // nnodes * WNodeLayout<W>::kBytes
   DevTri* d_tris = nullptr;     // WBVH: leaf order; kd: triangle-ID order
@@ -131,6 +132,7 @@ struct MultiLaunch {
   int predicate = 0;
   int device = 0;
   int stack_depth = 8;  // deepest scene's tree depth
+  bool wait = false;    // most rays lie in scenes of few tests per visit (see many_rays)
   uint32_t* d_counter = nullptr;
   uint32_t* d_status = nullptr;
   // optional: one status word per batch (a ray's loop-bound stop is recorded
@@ -164,6 +166,13 @@ void build_kd_reference(const float* tri_verts, uint32_t ntris, KdHost* out);
 // same tree shape) and rewrites its triangle records.
 void refit_wbvh(WBVHHost* h, const float* tri_verts, uint32_t ntris);
 void make_dev_tris(const float* tri_verts, uint32_t ntris, const uint32_t* order, DevTri* out);
+// Triangle tests per node visit that a random ray is expected to make in a tree
+// of width 8: the surface area of the leaves' boxes times their triangles over
+// that of the nodes' (the SAH's estimate).  A choice of kernel form, nothing
+// else, so a refit leaves it as it was.
+float tests_per_visit(const WBVHHost& h);
+constexpr float kFewTests = 0.55f;       // trace.cu: many_rays
+constexpr float kFewTestsMulti = 1.2f;  // ... in a multi-scene launch
 // How far triangle boxes are padded in a scene of these bounds: 1e-5 of the
 // larger of its extent and its largest coordinate.
 float box_pad(const float lo[3], const float hi[3], float maxabs);

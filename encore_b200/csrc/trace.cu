@@ -1546,10 +1546,17 @@ constexpr int kFewWarps = 32;
 bool few_rays(const Launch& L, size_t n, int sms) {
   return !L.fixed_chunk && !L.fixed_shape && n <= (size_t)sms * kFewWarps * 4;
 }
-// Launches long enough for WAIT to pay: six chunks of 32 rays per resident warp
-// (1,022,976 rays).  At 300,000 / 524,288 / 1M / 2M / 4M eye and bounce rays on
-// 10,000 to 100,000 triangles it took 315 / 225 / 342 / 584 / 1,060 us against 305 /
-// 222 / 343 / 592 / 1,083 without.
+// Whether WAIT pays: a launch of six chunks of 32 rays per resident warp or more
+// (1,022,976 rays), in a tree with fewer than kFewTests triangle tests per node
+// visit.  At 300,000 / 524,288 / 1M / 2M / 4M eye rays on 10,000 random triangles
+// (0.34 tests) it took 315 / 225 / 340 / 580 / 1,056 us against 305 / 222 / 343 / 592 /
+// 1,083 without.  Where a visit tests more, rounds are fuller anyway: 1.84M bounce
+// rays on 100,000 random triangles (1.05) took 480 us against 468, 4M on 1M (2.1)
+// 6,210 against 6,049; fields of 20,000 to 2M triangles lie at 0.36 to 0.51 and gain
+// 1.4 to 6 %.  The multi-scene form, whose 64 registers hold the waiting lanes'
+// state at no cost, gains up to kFewTestsMulti: 3M rays over two scenes 721 -> 685
+// us on a 131,072-triangle field, 1,234 -> 1,197 / 1,441 -> 1,404 / 1,869 -> 1,851 on
+// 10,000 / 30,000 / 100,000 random triangles, 4,920 -> 5,015 on 1M.
 bool many_rays(size_t n, int blocks, int threads) {
   return n >= (size_t)blocks * (size_t)threads * 6;
 }
@@ -1604,7 +1611,7 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
     else if (ord) k = wbvh_trace<W, CLAMP, false, COUNT, false, false, true>;
     if constexpr (W == 8 && !COUNT) {
       const int blocks = sms * (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksClosest);
-      if (!lane && many_rays(n, blocks, L.block))
+      if (!lane && a.tests_per_visit < kFewTests && many_rays(n, blocks, L.block))
         k = ord ? wbvh_trace<W, CLAMP, false, false, false, false, true, true>
                 : wbvh_trace<W, CLAMP, false, false, false, false, false, true>;
     }
@@ -1816,7 +1823,7 @@ int launch_multi_w(const MultiLaunch& m, const Launch& L, cudaStream_t s) {
   if constexpr (W == 8 && !ANY) {
     const int blocks = device_sm_count(m.device) *
                        (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksMulti);
-    if (many_rays(m.total, blocks, L.block))
+    if (m.wait && many_rays(m.total, blocks, L.block))
       k = wbvh_trace<W, CLAMP, false, false, true, false, false, true>;
   }
   if (smem > 48 * 1024) {

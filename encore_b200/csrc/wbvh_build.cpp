@@ -528,6 +528,43 @@ bool refit_levels_of(const WBVHHost& h, std::vector<uint32_t>& start) {
                       : (h.width == 4 ? levels_w<4>(h, start) : levels_w<8>(h, start));
 }
 
+float tests_per_visit(const WBVHHost& h) {
+  using L = WNodeLayout<8>;
+  if (h.width != 8) return 1.f;
+  double visits = 0.0, tests = 0.0;
+  for (uint32_t i = 0; i < h.nnodes; ++i) {
+    const uint8_t* raw = h.nodes.data() + (size_t)i * L::kBytes;
+    WNodeHeader hd;
+    std::memcpy(&hd, raw, sizeof(hd));
+    double step[3], lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+      step[a] = std::ldexp(1.0, (int)hd.e[a] - 127);
+      lo[a] = 255.0;
+      hi[a] = 0.0;
+    }
+    auto area = [&](const double* x, const double* y) {
+      double e[3];
+      for (int a = 0; a < 3; ++a) e[a] = std::max(0.0, y[a] - x[a]) * step[a];
+      return e[0] * e[1] + e[1] * e[2] + e[2] * e[0];
+    };
+    for (int c = 0; c < 8; ++c) {
+      const uint32_t m = raw[L::kMetaOff + c];
+      if (m == 0) continue;
+      double x[3], y[3];
+      for (int a = 0; a < 3; ++a) {
+        x[a] = raw[L::kQOff + a * 8 + c];
+        y[a] = raw[L::kQOff + (3 + a) * 8 + c];
+        lo[a] = std::min(lo[a], x[a]);
+        hi[a] = std::max(hi[a], y[a]);
+      }
+      if (m < 32) visits += area(x, y);
+      else tests += area(x, y) * (m >> 5);
+    }
+    if (i == 0) visits += area(lo, hi);
+  }
+  return visits > 0.0 ? (float)(tests / visits) : 1.f;
+}
+
 void build_wbvh(const float* tri_verts, uint32_t ntris, int width, int max_leaf, WBVHHost* out) {
   if (ntris == 0) throw std::runtime_error("empty scene");
   if (max_leaf < 1 || max_leaf > 4) throw std::runtime_error("max_leaf_tris must be 1..4");

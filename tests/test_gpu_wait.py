@@ -43,6 +43,7 @@ def test_long_launches_match_short_ones(gpu, predicate, extra):
     alone = torch.full((m, 4), 7, dtype=torch.int32, device="cuda")
     other.intersect_device(d, m, alone)
     h = [torch.full((k, 4), 7, dtype=torch.int32, device="cuda") for k in (n // 2, n - n // 2, m)]
+    # (most rays lie in a scene whose launches are of this form)
     b = BatchLaunch([(acc, rays[:n // 2], h[0]), (acc, rays[n // 2:].contiguous(), h[1]), (other, d, h[2])])
     b.launch()
     b.check()
