@@ -115,6 +115,17 @@ cudaMemPool_t map_pool(int device, bool create) {
   return g_pool[device];
 }
 
+// An allocation from the pool of the current device `device` (cudaMalloc where
+// it has none), on the legacy default stream.
+cudaError_t pool_alloc(void** p, size_t bytes, int device, bool* pooled) {
+  cudaMemPool_t pool = map_pool(device, true);
+  *pooled = pool && cudaMallocFromPoolAsync(p, bytes, pool, 0) == cudaSuccess;
+  if (*pooled) return cudaSuccess;
+  cudaGetLastError();
+  *p = nullptr;
+  return device_malloc(p, bytes);
+}
+
 // Gives the device back what its pool keeps.
 void trim_map_pool(int device) {
   if (cudaMemPool_t pool = map_pool(device, false)) cudaMemPoolTrimTo(pool, 0);
@@ -1123,17 +1134,12 @@ cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
                rec = 16 * (size_t)d.n;
   const size_t o_build = o_pos + up(3 * rec);
   const size_t bytes = o_build + scratch + 256;
-  cudaMemPool_t pool = map_pool(d.device, true);
-  // on the legacy default stream, where the map is then written; its creation
-  // waits for that, so the map may be used on any stream
-  d.pooled = pool && cudaMallocFromPoolAsync(&d.slab, bytes, pool, 0) == cudaSuccess;
-  if (!d.pooled) {
-    cudaGetLastError();
-    cudaError_t e = device_malloc(&d.slab, bytes);
-    if (e != cudaSuccess) {
-      d.slab = nullptr;
-      return e;
-    }
+  // The map is then written on the stream of this allocation, and its creation
+  // waits for that, so it may be used on any stream.
+  const cudaError_t e = pool_alloc(&d.slab, bytes, d.device, &d.pooled);
+  if (e != cudaSuccess) {
+    d.slab = nullptr;
+    return e;
   }
   char* base = static_cast<char*>(d.slab);
   d.d_counter = reinterpret_cast<uint32_t*>(base);
@@ -1229,7 +1235,9 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   bool direct = on_device && build;
   for (int i = 0; i < 3 && direct; ++i) direct = readable_on(src[i], bytes, device);
   void* work = nullptr;
-  if (e == cudaSuccess && build && !direct && device_malloc(&work, 3 * bytes) != cudaSuccess) {
+  bool work_pooled = false;
+  if (e == cudaSuccess && build && !direct &&
+      pool_alloc(&work, 3 * bytes, device, &work_pooled) != cudaSuccess) {
     cudaGetLastError();
     work = nullptr;
     build = false;
@@ -1258,7 +1266,8 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   } else if (e == cudaSuccess) {
     e = host_photon_map(src[0], src[1], src[2], d, what);
   }
-  cudaFree(work);
+  if (work_pooled) cudaFreeAsync(work, 0);  // after the build, which used that stream
+  else cudaFree(work);
   if (e != cudaSuccess) {
     free_photon_map(d);
     delete m;

@@ -12,6 +12,7 @@
 //      only the count of right-going photons before it in the list: the ranges
 //      of a level have two sizes, so the count at a range's start has a closed
 //      form.
+//      Ranges of at most 1,024 photons are split to the leaves in shared memory.
 //   3. The records are written leaf by leaf from the x list, and the boxes
 //      formed from them.
 //
@@ -19,9 +20,10 @@
 // photons inside a leaf and on equal coordinates, neither of which a k-nearest
 // set depends on.
 //
-// What bounds it: some 65 short launches (three per level) of a few
-// microseconds, each streaming 4 to 24 bytes per photon and axis through L2.
-// 500,000 photons: 44.9 ms on the host, 0.63 ms here.
+// What bounds it: some 50 short launches (18 for the sort, three per level) of a
+// few microseconds, each streaming 4 to 24 bytes per photon and axis through L2.
+// 500,000 photons: 44.9 ms on the host, 0.63 ms here with a launch triple for every
+// level, 0.51 with the last five in shared memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -190,6 +192,14 @@ __device__ __forceinline__ Range range_of(uint32_t n, int level, uint32_t p) {
   return r;
 }
 
+// The right-going photons of the ranges before g, in a level whose range sizes
+// are q and q + 1: a range of size z sends (z + 1) / 2 right, so they sent
+// (g.b + how many of them are odd) / 2; g.b - g.s * q of them have size q + 1.
+__device__ __forceinline__ uint32_t ones_before(const Range& g, uint32_t q) {
+  const uint32_t big = g.b - g.s * q;
+  return (g.b + ((q & 1u) ? g.s - big : big)) / 2;
+}
+
 // The side of every photon at this level: 1 beyond the median of its range in
 // the list of the range's widest axis.
 __global__ void __launch_bounds__(kThreads) split_side(const float* __restrict__ pos,
@@ -279,13 +289,87 @@ __global__ void __launch_bounds__(kThreads) split_move(const uint32_t* __restric
     const uint32_t p = blockIdx.x * kTile + r * kThreads + threadIdx.x;
     if (p >= n) continue;
     const Range g = range_of(n, level, p);
-    // A range of size z sends (z + 1) / 2 right, so the ranges before this one
-    // sent (b + how many of them are odd) / 2; b - s * q of them have size q + 1.
-    const uint32_t big = g.b - g.s * q;
-    const uint32_t odd = (q & 1u) ? g.s - big : big;
-    const uint32_t ones = before + s_row[r * kWarps + warp] + in_row[r] - (g.b + odd) / 2;
+    const uint32_t ones = before + s_row[r * kWarps + warp] + in_row[r] - ones_before(g, q);
     out[(size_t)blockIdx.y * n + ((right >> r) & 1u ? g.m + ones : p - ones)] = id[r];
   }
+}
+
+// The levels below `top` in shared memory: one block per range of at most kRange
+// photons, its three lists as places in its x list.  `inv` (one word per photon)
+// takes the photons' places in that list.  order: the photons of the last level.
+constexpr uint32_t kRange = 1024;
+constexpr int kPer = kRange / kThreads;  // consecutive list places per thread
+__global__ void __launch_bounds__(kThreads) split_ranges(const float* __restrict__ pos,
+                                                         const uint32_t* lists, uint32_t* inv,
+                                                         uint32_t n, int top, int depth,
+                                                         uint32_t* order) {
+  __shared__ float s_pos[3][kRange];
+  __shared__ uint32_t s_id[kRange], s_warp[kWarps];
+  __shared__ uint16_t s_list[2][3][kRange];
+  __shared__ uint8_t s_side[kRange];
+  uint32_t b = 0, e = n;
+  for (int l = top - 1; l >= 0; --l) {
+    const uint32_t m = b + (e - b) / 2;
+    if ((blockIdx.x >> l) & 1u) b = m;
+    else e = m;
+  }
+  const uint32_t c = e - b;
+  for (uint32_t i = threadIdx.x; i < c; i += kThreads) {
+    const uint32_t id = lists[b + i];
+    s_id[i] = id;
+    inv[id] = i;
+    s_list[0][0][i] = (uint16_t)i;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) s_pos[a][i] = __ldg(pos + 3 * (size_t)id + a);
+  }
+  __syncthreads();
+  for (int a = 1; a < 3; ++a)
+    for (uint32_t i = threadIdx.x; i < c; i += kThreads)
+      s_list[0][a][i] = (uint16_t)inv[lists[(size_t)a * n + b + i]];
+  __syncthreads();
+  int cur = 0;
+  for (int level = top; level < depth; ++level, cur ^= 1) {
+    Range g[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t p = kPer * threadIdx.x + j;
+      if (p >= c) continue;
+      g[j] = range_of(c, level - top, p);
+      float ext[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        ext[a] = s_pos[a][s_list[cur][a][g[j].e - 1]] - s_pos[a][s_list[cur][a][g[j].b]];
+      int axis = 0;
+      if (ext[1] > ext[0]) axis = 1;
+      if (ext[2] > (axis == 1 ? ext[1] : ext[0])) axis = 2;
+      s_side[s_list[cur][axis][p]] = p >= g[j].m ? 1 : 0;
+    }
+    __syncthreads();
+    const uint32_t q = c >> (level - top);
+    const int nlists = level == depth - 1 ? 1 : 3;
+    for (int a = 0; a < nlists; ++a) {
+      uint32_t id[kPer], one[kPer], sum = 0, total;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        const uint32_t p = kPer * threadIdx.x + j;
+        id[j] = p < c ? s_list[cur][a][p] : 0u;
+        one[j] = p < c ? s_side[id[j]] : 0u;
+        sum += one[j];
+      }
+      uint32_t before = block_scan(sum, s_warp, &total);
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        const uint32_t p = kPer * threadIdx.x + j;
+        if (p < c) {
+          const uint32_t ones = before - ones_before(g[j], q);
+          s_list[cur ^ 1][a][one[j] ? g[j].m + ones : p - ones] = (uint16_t)id[j];
+        }
+        before += one[j];
+      }
+    }
+    __syncthreads();
+  }
+  for (uint32_t i = threadIdx.x; i < c; i += kThreads) order[b + i] = s_id[s_list[cur][0][i]];
 }
 
 // The bounds of a warp's 32 boxes to item j of a level's arrays.
@@ -404,14 +488,15 @@ int build_photon_device(const float* pos, const float* nrm, const float* pw, con
       sort_move<<<tg, kThreads>>>(pos, in, n, pass, hist, sums, items[pass & 1],
                                   pass == kPasses - 1 ? lists[0] : nullptr);
     }
-    int cur = 0;
-    for (int level = 0; level < d.depth; ++level, cur ^= 1) {
-      const bool last = level == d.depth - 1;
-      const dim3 g((unsigned)tiles, last ? 1 : 3);
-      split_side<<<flat, kThreads>>>(pos, lists[cur], n, level, side);
-      split_count<<<g, kThreads>>>(lists[cur], side, n, hist);
-      split_move<<<g, kThreads>>>(lists[cur], side, n, level, hist, last ? order : lists[cur ^ 1]);
+    int cur = 0, top = 0;
+    while (((n + (1ull << top) - 1) >> top) > kRange) {
+      split_side<<<flat, kThreads>>>(pos, lists[cur], n, top, side);
+      split_count<<<tg, kThreads>>>(lists[cur], side, n, hist);
+      split_move<<<tg, kThreads>>>(lists[cur], side, n, top, hist, lists[cur ^ 1]);
+      cur ^= 1;
+      ++top;
     }
+    split_ranges<<<1u << top, kThreads>>>(pos, lists[cur], lists[cur ^ 1], n, top, d.depth, order);
   }
   write_leaves<<<(d.lvl_pad[0] + kWarps - 1) / kWarps, kThreads>>>(
       pos, nrm, pw, d.depth > 0 ? order : nullptr, n, d.depth, d.lvl_count[0], d.lvl_pad[0],
