@@ -973,9 +973,10 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
 // that is depends on neither).  The stack and the walk are wbvh_trace's for
 // width 8, child order, culling and the choice among candidates included, so the
 // hits are the same bits.  777 / 5,000 eye and bounce rays in 10,000 triangles: 49
-// / 66 us with a share of rays per warp, 33 / 43 us here (39 / 49 with the next
-// node fetched after the triangles); 777 shadow rays 58 -> 41.  Prefetching the
-// other children hit to L1 made 5,000 rays 2 us slower.
+// / 66 us with a share of rays per warp, 32 / 41 us here (39 / 49 with the next
+// node fetched after the triangles); 777 shadow rays 58 -> 37, four of them from
+// more than 64 registers.  Prefetching the other children hit to L1 made 5,000 rays
+// 2 us slower, loading the triangles ahead of the next node 4.
 
 // Position of the r-th set bit of m (r counted from 0, r < popc(m)), by
 // halving: keep the low half while it holds more than r set bits.
@@ -994,7 +995,7 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int r) {
 }
 
 template <bool CLAMP, bool ANY>
-__global__ void __launch_bounds__(128) wbvh_few(TraceParams P) {
+__global__ void __launch_bounds__(128, 4) wbvh_few(TraceParams P) {
   using L = WNodeLayout<8>;
   extern __shared__ uint2 s_stack[];
   const unsigned lane = threadIdx.x & 31u, grp = lane >> 3, c = lane & 7u;
@@ -1119,13 +1120,14 @@ __global__ void __launch_bounds__(128) wbvh_few(TraceParams P) {
           }
         }
       }
+      const unsigned cand = __ballot_sync(kFull, key != ~0ull);
       if (ANY) {
-        if ((__ballot_sync(kFull, key != ~0ull) >> (8 * grp)) & 0xffu) {
+        if ((cand >> (8 * grp)) & 0xffu) {
           hit_any = true;
           node = kNoItem;
           tris = 0;
         }
-      } else {
+      } else if (cand) {
         unsigned long long low = key;
 #pragma unroll
         for (int d = 1; d < 8; d <<= 1) {
@@ -1537,12 +1539,13 @@ unsigned ray_share(const Launch& L, size_t n, int sms, int* grid) {
   return (unsigned)share;
 }
 
-// The largest batch that wbvh_few takes, in warps of four rays per SM (18,944
-// rays on 148 SMs): at 19,000 rays it took 65 us against 79 in 10,000 random
-// triangles, 41 against 61 on a 131,072-triangle field and 70 against 99 for
-// shadow rays, at 38,000 rays 98 against 92, 62 against 70 and 103 against 99.  A
-// caller's choice of chunk, block or blocks per SM is one of wbvh_trace's shape.
-constexpr int kFewWarps = 32;
+// The largest batch that wbvh_few takes, in warps of four rays per SM (28,416
+// rays on 148 SMs): at 28,000 rays it took 82 us against 94 in 10,000 random
+// triangles, 47 against 59 on a 131,072-triangle field and 83 against 107 for
+// shadow rays in 100,000 triangles, at 38,000 rays 96 against 92, 62 against 70 and
+// 100 against 99.  A caller's choice of chunk, block or blocks per SM is one of
+// wbvh_trace's shape.
+constexpr int kFewWarps = 48;
 bool few_rays(const Launch& L, size_t n, int sms) {
   return !L.fixed_chunk && !L.fixed_shape && n <= (size_t)sms * kFewWarps * 4;
 }

@@ -36,8 +36,8 @@ def test_shared_out_batches_match_the_queue(gpu, scene, width, per_warp):
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     warps = sms * 16
-    n = {"1": 1, "31": 31, "33": 33, "warps": warps, "warps+1": warps + 1, "few": 128 * sms,
-         "few+1": 128 * sms + 1, "full": 32 * warps,
+    n = {"1": 1, "31": 31, "33": 33, "warps": warps, "warps+1": warps + 1, "few": 192 * sms,
+         "few+1": 192 * sms + 1, "full": 32 * warps,
          "full+1": 32 * warps + 1, "queue": 32 * 4 * 9 * sms + 1}[per_warp]
     rays = batch(n)
     acc = Accelerator("wbvh", width=width).build(scene)
