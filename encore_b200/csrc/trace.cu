@@ -350,8 +350,8 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   // 1,089 / 1,084 / 1,094 / 1,119 us (1,142 without WAIT), 4M eye rays on 10,000
   // triangles 1,096 / 1,111 / 1,095 / 1,080 / 1,070 / 1,060 / 1,065 / 1,080 (1,083), 16
   // scenes in one launch 1,136 / 1,147 / 1,135 / 1,124 / 1,115 / 1,105 / 1,108 / 1,131
-  // (1,135).  Any hit gains 6 % where few rays are blocked and loses 2 % where
-  // half are, so it does without.
+  // (1,135); any hit at 4 / 6 / 8 / 12 lanes: 2M rays over a field 298 / - / 286 / 290
+  // (305 without), 2M on 10,000 triangles - / 723 / 714 / - (721).
   static_assert(!WAIT || kCoop, "the per-lane form has no triangle rounds");
   constexpr int kWait = 8;
   // the per-lane form keeps the group bound (without it ptxas spills more)
@@ -1520,7 +1520,8 @@ constexpr size_t stack_entry_bytes(int W) {
 // Warps per SM that a batch smaller than one grid of 32-ray chunks is spread
 // over.  Such a launch lasts as long as its slowest warp, and a warp with
 // fewer rays steps faster (fewer triangle rounds, fewer divergent refills),
-// while more warps slow one another down.  777 eye rays on 10,000 triangles:
+// while more warps slow one another down.  With this kernel (width 8 hands up to
+// 28,416 rays to wbvh_few, below), 777 eye rays on 10,000 triangles took
 // 76 us with 32 rays per warp on every resident warp's queue, 49 us at 16;
 // 20,000 rays: 104 us, and 84 / 80 / 88 / 106 us at 8 / 12 / 16 / 36; 100,000
 // rays: 153 us, 117 us at 8 to 16 (32 rays per warp, fewer blocks).
@@ -1556,7 +1557,10 @@ bool few_rays(const Launch& L, size_t n, int sms) {
 // 1,083 without.  Where a visit tests more, rounds are fuller anyway: 1.84M bounce
 // rays on 100,000 random triangles (1.05) took 480 us against 468, 4M on 1M (2.1)
 // 6,210 against 6,049; fields of 20,000 to 2M triangles lie at 0.36 to 0.51 and gain
-// 1.4 to 6 %.  The multi-scene form, whose 64 registers hold the waiting lanes'
+// 1.4 to 6 %.  Any hit, at 9 blocks per SM too: 4M / 2M / 1M rays over fields 666 ->
+// 607 / 305 -> 286 / 164 -> 160 us, 2M on 2,000 / 10,000 / 20,000 random triangles
+// 446 -> 434 / 721 -> 714 / 757 -> 753, 1.5M on 100,000 656 -> 669; 300,000 rays 62 ->
+// 64.  The multi-scene form, whose 64 registers hold the waiting lanes'
 // state at no cost, gains up to kFewTestsMulti: 3M rays over two scenes 721 -> 685
 // us on a 131,072-triangle field, 1,234 -> 1,197 / 1,441 -> 1,404 / 1,869 -> 1,851 on
 // 10,000 / 30,000 / 100,000 random triangles, 4,920 -> 5,015 on 1M.
@@ -1612,11 +1616,15 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
   if constexpr (!ANY) {
     if (lane) k = wbvh_trace<W, CLAMP, false, COUNT, false, true, true>;
     else if (ord) k = wbvh_trace<W, CLAMP, false, COUNT, false, false, true>;
-    if constexpr (W == 8 && !COUNT) {
-      const int blocks = sms * (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksClosest);
-      if (!lane && a.tests_per_visit < kFewTests && many_rays(n, blocks, L.block))
-        k = ord ? wbvh_trace<W, CLAMP, false, false, false, false, true, true>
-                : wbvh_trace<W, CLAMP, false, false, false, false, false, true>;
+  }
+  if constexpr (W == 8 && !COUNT) {
+    const int blocks =
+        sms * (L.blocks_per_sm > 0 ? L.blocks_per_sm : (ANY ? kBlocksAny : kBlocksClosest));
+    if (!lane && a.tests_per_visit < kFewTests && many_rays(n, blocks, L.block)) {
+      k = wbvh_trace<W, CLAMP, ANY, false, false, false, false, true>;
+      if constexpr (!ANY) {
+        if (ord) k = wbvh_trace<W, CLAMP, false, false, false, false, true, true>;
+      }
     }
   }
   if (smem > 48 * 1024) {

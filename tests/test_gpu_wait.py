@@ -66,3 +66,28 @@ def test_stack_limit_is_reported_by_long_launches(gpu):
         acc.check()
     assert ei.value.status == 4
     assert (hits[:, 0] >= -1).all() and (hits[:, 0] < 3000).all()
+
+
+@pytest.mark.parametrize("scene", ["soup", "field"])
+@pytest.mark.parametrize("extra", [-1, 0, 70_001])
+def test_long_any_hit_launches_match_short_ones(gpu, scene, extra):
+    """Any hit takes the same form at the same size; the short launches'
+    answers are those of a form without waiting."""
+    import torch
+    tris = (scenes.random_triangles(3000, seed=117, scale=SCALE) if scene == "soup"
+            else scenes.heightfield(res=96, seed=118, scale=SCALE))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = sms * 9 * 128 * 6 + extra
+    base = scenes.random_sphere_rays(200_003, seed=119, hi=(SCALE, SCALE, SCALE))
+    base[::3, 7] = 0.2 * SCALE  # bounded segments between unbounded rays
+    d = torch.from_numpy(base).cuda()
+    m = len(base)
+    acc = Accelerator("wbvh").build(tris)
+    short = torch.full((m,), 7, dtype=torch.uint8, device="cuda")
+    acc.occluded_device(d, m, short)
+    assert 0.02 * m < int((short == 1).sum()) < 0.98 * m
+    pick = torch.randint(0, m, (n,), device="cuda", generator=torch.Generator("cuda").manual_seed(6))
+    occ = torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+    acc.occluded_device(d[pick].contiguous(), n, occ)
+    acc.check()
+    assert torch.equal(occ, short[pick])
