@@ -351,9 +351,12 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
   // triangles 1,096 / 1,111 / 1,095 / 1,080 / 1,070 / 1,060 / 1,065 / 1,080 (1,083), 16
   // scenes in one launch 1,136 / 1,147 / 1,135 / 1,124 / 1,115 / 1,105 / 1,108 / 1,131
   // (1,135); any hit at 4 / 6 / 8 / 12 lanes: 2M rays over a field 298 / - / 286 / 290
-  // (305 without), 2M on 10,000 triangles - / 723 / 714 / - (721).
+  // (305 without), 2M on 10,000 triangles - / 723 / 714 / - (721).  The step asks only
+  // how many lanes are at leaves: a second ballot, for whether any other walks, took
+  // the heightfield's rays 1,079 us (1,066 now) and the 16 scenes 1,100 (1,095).
   static_assert(!WAIT || kCoop, "the per-lane form has no triangle rounds");
   constexpr int kWait = 8;
+  static_assert(kWait + kRefill <= 32, "a warp that waits has lanes that walk");
   // the per-lane form keeps the group bound (without it ptxas spills more)
   constexpr bool kBound = kGroupBound || LANE;
   // L2 priorities in the single-scene cooperative closest-hit form only: in
@@ -792,8 +795,9 @@ __global__ void __launch_bounds__(128, ANY    ? kBlocksAny
     // "t < best_t, or equal t and a lower ID", whatever the order.
     {
       unsigned pend = __ballot_sync(kFull, tmask != 0);
-      if (WAIT && !exhausted && __popc(pend) < kWait && pend != __ballot_sync(kFull, ray >= 0))
-        pend = 0;
+      // (while the queue has rays, fewer than kRefill lanes are idle here, so with
+      // fewer than kWait at leaves others still walk)
+      if (WAIT && !exhausted && __popc(pend) < kWait) pend = 0;
       const unsigned wib = threadIdx.x >> 5;
       uint32_t* it_tri = s_coop_tri + wib * 32;
       uint32_t* it_own = s_coop_own + wib * 32;
@@ -1558,9 +1562,10 @@ bool few_rays(const Launch& L, size_t n, int sms) {
 // rays on 100,000 random triangles (1.05) took 480 us against 468, 4M on 1M (2.1)
 // 6,210 against 6,049; fields of 20,000 to 2M triangles lie at 0.36 to 0.51 and gain
 // 1.4 to 6 %.  Any hit, at 9 blocks per SM too: 4M / 2M / 1M rays over fields 666 ->
-// 607 / 305 -> 286 / 164 -> 160 us, 2M on 2,000 / 10,000 / 20,000 random triangles
+// 609 / 305 -> 288 / 164 -> 160 us, 2M on 2,000 / 10,000 / 20,000 random triangles
 // 446 -> 434 / 721 -> 714 / 757 -> 753, 1.5M on 100,000 656 -> 669; 300,000 rays 62 ->
-// 64.  The multi-scene form, whose 64 registers hold the waiting lanes'
+// 64; where no ray is blocked and most leave the field at once (4.18M toward a light
+// above it) 237 -> 242.  The multi-scene form, whose 64 registers hold the waiting lanes'
 // state at no cost, gains up to kFewTestsMulti: 3M rays over two scenes 721 -> 685
 // us on a 131,072-triangle field, 1,234 -> 1,197 / 1,441 -> 1,404 / 1,869 -> 1,851 on
 // 10,000 / 30,000 / 100,000 random triangles, 4,920 -> 5,015 on 1M.
