@@ -21,6 +21,9 @@ LIB = PKG / "libencore_b200.so"
 INCLUDE = PKG.parent / "include"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+# photon_build.cu calls the standard library's selection from device code, which is
+# constexpr, and so callable there, from C++20 on.
+STD = {"photon_build.cu": "-std=c++20"}
 
 
 def _nvcc() -> str:
@@ -43,7 +46,7 @@ def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
 
 def _compile(src: Path, obj: Path, nvcc: str, verbose_ptxas: bool) -> str:
     if src.suffix == ".cu":
-        cmd = [nvcc, *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
+        cmd = [nvcc, *ARCH, "-O3", "-lineinfo", STD.get(src.name, "-std=c++17"), "--expt-relaxed-constexpr",
                "-Xcompiler", "-fPIC,-O3", "-I", str(INCLUDE), "-c", str(src), "-o", str(obj)]
         if verbose_ptxas:
             cmd[1:1] = ["-Xptxas", "-v"]

@@ -1253,9 +1253,14 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
                      on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
       in[i] = to;
     }
+    bool refused = false;
     if (e == cudaSuccess)
-      e = (cudaError_t)build_photon_device(in[0], in[1], in[2], d, d.build);
-  } else if (e == cudaSuccess && on_device) {
+      e = (cudaError_t)build_photon_device(in[0], in[1], in[2], d, d.build, &refused);
+    if (refused) build = false;
+  }
+  if (build || e != cudaSuccess) {
+    // built, or nothing to build
+  } else if (on_device) {
     try {
       std::vector<float> h[3];
       for (int i = 0; i < 3 && e == cudaSuccess; ++i) {
@@ -1266,7 +1271,7 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
     } catch (const std::exception&) {
       e = cudaErrorMemoryAllocation;
     }
-  } else if (e == cudaSuccess) {
+  } else {
     e = host_photon_map(src[0], src[1], src[2], d, what);
   }
   if (work_pooled) cudaFreeAsync(work, 0);  // after the build, which used that stream

@@ -2,10 +2,12 @@
 //
 // Replaces PhotonMap::BalanceAndConstruct (PhotonMap.cpp:167-221).  The
 // reference keeps one photon per node and picks the split axis from a running
-// box that starts at +-1e10 (PhotonMap.cpp:27-28, 182-191); the result of a
-// k-nearest query does not depend on the tree, so this build uses bucketed
+// box that starts at +-1e10 (PhotonMap.cpp:27-28, 182-191); the distances of a
+// k-nearest query do not depend on the tree, so this build uses bucketed
 // leaves of 32 photons and the range's largest extent, which is what a warp
-// gather wants.
+// gather wants.  Which of several photons at the same k-th distance a gather
+// keeps does depend on it, down to the order inside a leaf: the device build
+// (photon_build.cu) makes this tree, photon for photon.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -16,6 +18,9 @@
 
 namespace enc {
 namespace {
+
+// A coordinate as the splits order it: not-a-numbers last, with the infinite.
+inline float split_coord(float c) { return std::isnan(c) ? INFINITY : c; }
 
 struct TreeBuilder {
   const float* pos;
@@ -45,7 +50,9 @@ struct TreeBuilder {
     uint32_t m = b + (e - b) / 2;
     if (e > b) {
       std::nth_element(idx.begin() + b, idx.begin() + m, idx.begin() + e,
-                       [&](uint32_t p, uint32_t q) { return pos[3 * (size_t)p + axis] < pos[3 * (size_t)q + axis]; });
+                       [&](uint32_t p, uint32_t q) {
+                         return split_coord(pos[3 * (size_t)p + axis]) < split_coord(pos[3 * (size_t)q + axis]);
+                       });
     }
     nd.axis = axis;
     nd.split = (m < e) ? pos[3 * (size_t)idx[m] + axis] : 0.f;

@@ -87,11 +87,14 @@ void photon_layout(size_t n, DevPhotonMap* d);
 
 // Device build (photon_build.cu) of a map whose arrays are allocated, from
 // n >= 1 photons in device memory (3 floats each per photon, outside the map's
-// arrays).  `scratch`: photon_build_scratch(n) bytes, 256-byte aligned.  On the legacy default stream; waits for it.
-// Returns a CUDA error code; d.device must be current.
+// arrays): the records of build_photon_tree in the same order.  `scratch`:
+// photon_build_scratch(n) bytes, 256-byte aligned.  On the legacy default stream;
+// waits for it.  *refused: the photons need a selection that only the host build
+// makes (coordinates on which nth_element's partitions stay lopsided).  Returns
+// a CUDA error code; d.device must be current.
 size_t photon_build_scratch(size_t n);
 int build_photon_device(const float* d_pos, const float* d_nrm, const float* d_pow,
-                        const DevPhotonMap& d, void* scratch);
+                        const DevPhotonMap& d, void* scratch, bool* refused);
 
 // Launchers (gather.cu).  k <= 256.  Asynchronous on `stream`.
 int launch_radiance(const DevPhotonMap& m, const float* d_qpos, const float* d_qnrm, size_t nq,

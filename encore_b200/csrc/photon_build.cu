@@ -1,42 +1,85 @@
-// Device build of the photon tree (layout in photon.h): the host build's tree
-// shape -- every range split at its median index on the axis of its largest
-// extent, leaves of at most 32 photons, 32-ary boxes above them -- formed level
-// by level from three sorted lists.
+// Device build of the photon tree (layout in photon.h): the host build's tree,
+// photon for photon.  Every range is split at its median index on the axis of its
+// largest extent by what std::nth_element does there, so the order of equal
+// coordinates and of the photons inside a leaf is the host's as well: of photons
+// at equal distances a gather keeps those it meets first, and which it meets
+// first must not depend on where the map was made.
 //
-//   1. The photons are sorted along x, y and z: stable 8-bit counting passes
-//      over order-preserving keys, the three axes side by side.
-//   2. For each level of the tree: in the list of its split axis, a range's
-//      photons at and beyond the median position go right; every list is then
-//      split stably, so it stays sorted inside each new range.  A range's extent
-//      is the distance of its list's ends, and its place after the split needs
-//      only the count of right-going photons before it in the list: the ranges
-//      of a level have two sizes, so the count at a range's start has a closed
-//      form.
-//      Ranges of at most 1,024 photons are split to the leaves in shared memory.
-//   3. The records are written leaf by leaf from the x list, and the boxes
-//      formed from them.
+// The algorithm is introselect (Musser 1997): while more than three elements are
+// left, a pivot -- the median of the second, the middle and the last element --
+// goes to the front, the others are partitioned about it as Hoare does, and the
+// search goes on in the part that holds the median; after 2 log2(n) partitions a
+// heap selects instead.  Only the partitions are done in parallel.  Hoare's
+// pointers stop, from the left, at the elements that are not smaller than the
+// pivot and, from the right, at those that are not larger; they exchange the m-th
+// of the one with the m-th of the other while it lies to its left.  So an element's
+// partner follows from the count of the first kind before it and of the second
+// behind it.  What remains (three elements, or the heap) is the library's own
+// code.
 //
-// The tree differs from the host build's (nth_element) only in the order of
-// photons inside a leaf and on equal coordinates, neither of which a k-nearest
-// set depends on.
+//   * Ranges of more than kShared photons: one cluster of blocks per range narrows
+//     the selection in device memory, and its first block ends it in shared memory
+//     (split_cluster).
+//   * Down to kLeafRange photons: one block per range, in shared memory
+//     (split_block).
+//   * The levels below that: one launch, one block per such range, its warps in
+//     teams of one per range of a level (split_ranges).
+//   * The records are written leaf by leaf, and the boxes formed from them.
 //
-// What bounds it: some 50 short launches (18 for the sort, three per level) of a
-// few microseconds, each streaming 4 to 24 bytes per photon and axis through L2.
-// 500,000 photons: 44.9 ms on the host, 0.63 ms here with a launch triple for every
-// level, 0.51 with the last five in shared memory.
+// What bounds it: the length of the chain.  A level takes some eight to fifteen
+// partitions, one after another, of about 2,000 cycles in a block (four barriers,
+// and little between them) and 17,000 to 40,000 in a cluster.  500,000 photons: 45 ms
+// on the host, 0.94 ms here, 0.55 of them in the five levels of split_cluster, 0.17
+// in the four of split_block and 0.07 in split_ranges (clusters of 16 blocks: no
+// faster; rounds of launches over the whole device in their place: 1.42 ms; fewer
+// warps as a block's range shrinks: no faster).  A build that sorts the photons
+// along each axis once and splits the lists took 0.51 ms, but orders equal
+// coordinates and a leaf's photons otherwise, and gathers with photons at equal
+// distances then differed.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 
 #include "engine.h"
 #include "photon.h"
+
+namespace cg = cooperative_groups;
 
 namespace enc {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kThreads = 256, kRows = 8, kWarps = kThreads / 32;
-constexpr uint32_t kTile = kThreads * kRows;
+constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr uint32_t kTile = 2048;  // photons of a range that one block of range_extent takes
+constexpr int kBlock = 1024;      // threads of the kernels with one block or cluster per range
+constexpr unsigned kCluster = 8;  // blocks per cluster
+// Elements that a block holds: 8 bytes each, and 2 for the partition's lists.
+constexpr uint32_t kShared = 22528;
+constexpr size_t kElemBytes = sizeof(float) + sizeof(uint32_t) + sizeof(uint16_t);
+constexpr uint32_t kLeafRange = 1024;
+// Elements left from which one warp goes on alone: a partition by a team costs it
+// four barriers.
+constexpr uint32_t kWarpRange = 128;
+// A heap over more elements than this is left to the host build.
+constexpr uint32_t kMostHeap = 2048;
+
+// An element of a selection: the photon's coordinate on the split axis, and the
+// photon.  Its assignment is its own, so the library shifts elements one by one;
+// a memmove between overlapping places of shared memory came out wrong.
+struct alignas(8) Elem {
+  float key;
+  uint32_t id;
+  constexpr Elem& operator=(const Elem& o) {
+    key = o.key;
+    id = o.id;
+    return *this;
+  }
+};
+struct KeyLess {
+  constexpr bool operator()(const Elem& a, const Elem& b) const { return a.key < b.key; }
+};
 
 __device__ __forceinline__ unsigned lt_mask() {
   unsigned m;
@@ -47,329 +90,515 @@ __device__ __forceinline__ uint32_t coord_key(float f) {
   const uint32_t b = __float_as_uint(f);
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
-// Item i of an axis's list (key, photon) and its digit in counting pass `pass`.
-// Passes 0 and 1 sort by the upper half of the next axis's key, passes 2 to 5 by
-// the axis's own key, so photons of equal coordinate -- a wall's -- are ordered
-// along the wall and a split among them parts it instead of halving its density
-// (a k = 50 gather in a room tested 183 photons a query with the ties in photon
-// order, 159 with this).
-constexpr int kPasses = 6;
-struct Item {
-  uint2 v;
-  uint32_t digit;
+__device__ __forceinline__ float of_key(uint32_t k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+// The coordinate a photon is split by (photon.cpp: split_coord).
+__device__ __forceinline__ float split_coord(const float* pos, uint32_t id, int axis) {
+  const float c = __ldg(pos + 3 * (size_t)id + axis);
+  return isnan(c) ? INFINITY : c;
+}
+
+// The extents of a range of photons as six keys that are all maxima: the complement
+// of the smallest coordinate's key and the largest one's, per axis; not-a-numbers
+// left out.  An empty axis is (+inf, -inf).
+struct Extent {
+  uint32_t nlo[3], hi[3];
 };
-__device__ __forceinline__ Item sort_item(const float* pos, const uint2* in, uint32_t n, int axis,
-                                          int pass, uint32_t i) {
-  Item it;
-  it.v = in ? in[(size_t)axis * n + i] : make_uint2(coord_key(__ldg(pos + 3 * (size_t)i + axis)), i);
-  const uint32_t key =
-      pass < 2 ? coord_key(__ldg(pos + 3 * (size_t)it.v.y + (axis == 2 ? 0 : axis + 1))) : it.v.x;
-  it.digit = (key >> (pass < 2 ? 16 + 8 * pass : 8 * (pass - 2))) & 255u;
-  return it;
-}
-
-// grid (tiles, 3): digit counts of each tile, hist[(axis * 256 + digit) * tiles + tile].
-__global__ void __launch_bounds__(kThreads) sort_count(const float* __restrict__ pos,
-                                                       const uint2* __restrict__ in, uint32_t n,
-                                                       int pass, uint32_t* hist) {
-  __shared__ uint32_t s_cnt[256];
-  const int axis = blockIdx.y;
-  s_cnt[threadIdx.x] = 0;
-  __syncthreads();
-  for (int r = 0; r < kRows; ++r) {
-    const uint32_t i = blockIdx.x * kTile + r * kThreads + threadIdx.x;
-    if (i < n) atomicAdd(&s_cnt[sort_item(pos, in, n, axis, pass, i).digit], 1u);
+__device__ __forceinline__ Extent no_extent() {
+  Extent x;
+  for (int a = 0; a < 3; ++a) {
+    x.nlo[a] = ~coord_key(INFINITY);
+    x.hi[a] = coord_key(-INFINITY);
   }
-  __syncthreads();
-  hist[(size_t)(axis * 256 + threadIdx.x) * gridDim.x + blockIdx.x] = s_cnt[threadIdx.x];
+  return x;
 }
-
-// Exclusive scan of one value per thread of a block of kThreads; total: the sum.
-__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t incl = v;
+__device__ __forceinline__ void grow(Extent& x, int a, float c) {
+  const bool no = isnan(c);
+  x.nlo[a] = max(x.nlo[a], no ? 0u : ~coord_key(c));
+  x.hi[a] = max(x.hi[a], no ? 0u : coord_key(c));
+}
+__device__ __forceinline__ void grow(Extent& x, const float* pos, uint32_t id) {
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t t = __shfl_up_sync(kFull, incl, d);
-    if ((int)lane >= d) incl += t;
-  }
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  uint32_t before = 0, sum = 0;
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) {
-    if (w < (int)warp) before += s_warp[w];
-    sum += s_warp[w];
-  }
-  __syncthreads();
-  *total = sum;
-  return before + incl - v;
-}
-
-// grid (256, 3): exclusive scan of one digit's tile counts; sums[axis * 256 + digit].
-__global__ void __launch_bounds__(kThreads) sort_scan(uint32_t* hist, uint32_t tiles,
-                                                      uint32_t* sums) {
-  __shared__ uint32_t s_warp[kWarps];
-  uint32_t* row = hist + (size_t)(blockIdx.y * 256 + blockIdx.x) * tiles;
-  uint32_t carry = 0;
-  for (uint32_t b = 0; b < tiles; b += kThreads) {
-    const uint32_t i = b + threadIdx.x;
-    uint32_t total;
-    const uint32_t x = block_scan(i < tiles ? row[i] : 0u, s_warp, &total);
-    if (i < tiles) row[i] = carry + x;
-    carry += total;
-  }
-  if (threadIdx.x == 0) sums[blockIdx.y * 256 + blockIdx.x] = carry;
-}
-
-// grid (tiles, 3): each tile's items to their places, in order.  A warp takes
-// kRows * 32 consecutive items; the lanes of a row with the same digit are
-// ranked by __match_any, rows and warps by running counts.
-__global__ void __launch_bounds__(kThreads) sort_move(const float* __restrict__ pos,
-                                                      const uint2* __restrict__ in, uint32_t n,
-                                                      int pass, const uint32_t* __restrict__ hist,
-                                                      const uint32_t* __restrict__ sums, uint2* out,
-                                                      uint32_t* list) {
-  __shared__ uint32_t s_cnt[kWarps][256], s_base[256], s_warp[kWarps];
-  const int axis = blockIdx.y;
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = lt_mask();
-  for (int w = 0; w < kWarps; ++w) s_cnt[w][threadIdx.x] = 0;
-  uint32_t total;
-  s_base[threadIdx.x] = block_scan(sums[axis * 256 + threadIdx.x], s_warp, &total) +
-                        hist[(size_t)(axis * 256 + threadIdx.x) * gridDim.x + blockIdx.x];
-  __syncthreads();
-  Item item[kRows];
-  uint32_t rank[kRows];
-  const uint32_t first = blockIdx.x * kTile + warp * (kRows * 32) + lane;
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const uint32_t i = first + r * 32;
-    item[r] = i < n ? sort_item(pos, in, n, axis, pass, i) : Item{make_uint2(0u, 0u), 256u};
-    const uint32_t digit = item[r].digit;
-    const unsigned peers = __match_any_sync(kFull, digit);
-    const int leader = __ffs(peers) - 1;
-    uint32_t old = 0;
-    if (i < n && (int)lane == leader) {
-      old = s_cnt[warp][digit];
-      s_cnt[warp][digit] = old + __popc(peers);
-    }
-    rank[r] = __shfl_sync(kFull, old, leader) + __popc(peers & lt);
-    __syncwarp();
-  }
-  __syncthreads();
-  {  // thread d: the places of digit d, warp by warp
-    uint32_t at = s_base[threadIdx.x];
-    for (int w = 0; w < kWarps; ++w) {
-      const uint32_t c = s_cnt[w][threadIdx.x];
-      s_cnt[w][threadIdx.x] = at;
-      at += c;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    if (first + r * 32 >= n) continue;
-    const size_t to = (size_t)axis * n + s_cnt[warp][item[r].digit] + rank[r];
-    if (list) list[to] = item[r].v.y;
-    else out[to] = item[r].v;
+  for (int a = 0; a < 3; ++a) {
+    grow(x, a, __ldg(pos + 3 * (size_t)id + a));
   }
 }
+__device__ __forceinline__ void warp_extent(Extent& x) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    x.nlo[a] = __reduce_max_sync(kFull, x.nlo[a]);
+    x.hi[a] = __reduce_max_sync(kFull, x.hi[a]);
+  }
+}
+__device__ __forceinline__ int widest(const Extent& x) {
+  float e[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) e[a] = __fsub_rn(of_key(x.hi[a]), of_key(~x.nlo[a]));
+  int axis = 0;
+  if (e[1] > e[0]) axis = 1;
+  if (e[2] > (axis == 1 ? e[1] : e[0])) axis = 2;
+  return axis;
+}
 
-// The range of the tree's level `level` that list position p lies in.
+// Range s of the tree's level `level`: [b, e), split at m.
 struct Range {
-  uint32_t b, m, e, s;  // [b, e) split at m; s: its index in the level
+  uint32_t b, m, e;
 };
-__device__ __forceinline__ Range range_of(uint32_t n, int level, uint32_t p) {
-  Range r{0u, 0u, n, 0u};
-  for (int l = 0; l < level; ++l) {
+__device__ __forceinline__ Range range_of(uint32_t n, int level, uint32_t s) {
+  Range r{0u, 0u, n};
+  for (int l = level - 1; l >= 0; --l) {
     const uint32_t m = r.b + (r.e - r.b) / 2;
-    const bool right = p >= m;
-    r.s = 2 * r.s + (right ? 1u : 0u);
-    if (right) r.b = m;
+    if ((s >> l) & 1u) r.b = m;
     else r.e = m;
   }
   r.m = r.b + (r.e - r.b) / 2;
   return r;
 }
 
-// The right-going photons of the ranges before g, in a level whose range sizes
-// are q and q + 1: a range of size z sends (z + 1) / 2 right, so they sent
-// (g.b + how many of them are odd) / 2; g.b - g.s * q of them have size q + 1.
-__device__ __forceinline__ uint32_t ones_before(const Range& g, uint32_t q) {
-  const uint32_t big = g.b - g.s * q;
-  return (g.b + ((q & 1u) ? g.s - big : big)) / 2;
+__device__ __forceinline__ int select_depth(uint32_t n) { return 2 * (31 - __clz((int)n)); }
+
+// Which of the places x, y, z holds the median of their keys x, y, z.
+__device__ __forceinline__ uint32_t median_place(uint32_t x, float kx, uint32_t y, float ky, uint32_t z,
+                                                 float kz) {
+  if (kx < ky) return ky < kz ? y : (kx < kz ? z : x);
+  return kx < kz ? x : (ky < kz ? z : y);
 }
 
-// The side of every photon at this level: 1 beyond the median of its range in
-// the list of the range's widest axis.
-__global__ void __launch_bounds__(kThreads) split_side(const float* __restrict__ pos,
-                                                       const uint32_t* __restrict__ lists,
-                                                       uint32_t n, int level, uint8_t* side) {
-  for (uint32_t p = blockIdx.x * kThreads + threadIdx.x; p < n; p += gridDim.x * kThreads) {
-    const Range r = range_of(n, level, p);
-    float ext[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const uint32_t* list = lists + (size_t)a * n;
-      ext[a] = __ldg(pos + 3 * (size_t)__ldg(list + r.e - 1) + a) -
-               __ldg(pos + 3 * (size_t)__ldg(list + r.b) + a);
+// ---------------------------------------------------------------------------
+// Partitions.  A team of warps -- one, some of a block, a block, a cluster -- has
+//   warps(), warp()   how many it has, and which of them the caller is;
+//   sync()            a barrier that also orders the team's memory accesses;
+//   offsets(ge, le)   of the counts of all its warps: the sum of `ge` over the
+//                     warps before the caller's, of `le` over those behind it;
+//   results(swaps, cut)  the sum and the minimum over its warps.
+// The last two are barriers too.
+
+struct WarpTeam {
+  __device__ unsigned warps() const { return 1; }
+  __device__ unsigned warp() const { return 0; }
+  __device__ void sync() const { __syncwarp(); }
+  __device__ void offsets(uint32_t& ge, uint32_t& le) const { ge = le = 0; }
+  __device__ void results(uint32_t&, uint32_t&) const { __syncwarp(); }
+};
+
+// What the warps of a block tell each other.
+struct TeamShared {
+  uint32_t ge[kBlock / 32], le[kBlock / 32], swaps[kBlock / 32], cut[kBlock / 32];
+  uint32_t all_ge, all_le, all_swaps, all_cut;  // of a block of a cluster
+};
+
+// `n` warps of a block, from warp `first` on; id: their barrier (0: the block's).
+struct BlockTeam {
+  unsigned n, first, id;
+  TeamShared& s;
+  __device__ unsigned warps() const { return n; }
+  __device__ unsigned warp() const { return (threadIdx.x >> 5) - first; }
+  __device__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n * 32) : "memory"); }
+  __device__ void put_counts(uint32_t ge, uint32_t le) const {
+    if ((threadIdx.x & 31u) == 0) {
+      s.ge[warp()] = ge;
+      s.le[warp()] = le;
     }
-    int axis = 0;
-    if (ext[1] > ext[0]) axis = 1;
-    if (ext[2] > (axis == 1 ? ext[1] : ext[0])) axis = 2;
-    side[__ldg(lists + (size_t)axis * n + p)] = p >= r.m ? 1 : 0;
+    sync();
   }
-}
-
-// grid (tiles, 3): photons of each tile that go right.
-__global__ void __launch_bounds__(kThreads) split_count(const uint32_t* __restrict__ lists,
-                                                        const uint8_t* __restrict__ side,
-                                                        uint32_t n, uint32_t* cnt) {
-  __shared__ uint32_t s_sum;
-  if (threadIdx.x == 0) s_sum = 0;
-  __syncthreads();
-  uint32_t c = 0;
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const uint32_t p = blockIdx.x * kTile + r * kThreads + threadIdx.x;
-    if (p < n) c += side[__ldg(lists + (size_t)blockIdx.y * n + p)];
+  __device__ void offsets(uint32_t& ge, uint32_t& le) const {
+    put_counts(ge, le);
+    const unsigned lane = threadIdx.x & 31u;
+    ge = __reduce_add_sync(kFull, lane < warp() ? s.ge[lane] : 0u);
+    le = __reduce_add_sync(kFull, lane > warp() && lane < n ? s.le[lane] : 0u);
   }
-  c = __reduce_add_sync(kFull, c);
-  if ((threadIdx.x & 31u) == 0 && c) atomicAdd(&s_sum, c);
-  __syncthreads();
-  if (threadIdx.x == 0) cnt[blockIdx.y * gridDim.x + blockIdx.x] = s_sum;
-}
-
-// grid (tiles, 3): the stable split of each list.
-__global__ void __launch_bounds__(kThreads) split_move(const uint32_t* __restrict__ lists,
-                                                       const uint8_t* __restrict__ side,
-                                                       uint32_t n, int level,
-                                                       const uint32_t* __restrict__ cnt,
-                                                       uint32_t* out) {
-  __shared__ uint32_t s_part[kWarps], s_row[kRows * kWarps];
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = lt_mask();
-  const uint32_t* list = lists + (size_t)blockIdx.y * n;
-  // right-going photons of the tiles before this one
-  uint32_t before = 0;
-  for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kThreads)
-    before += __ldg(cnt + blockIdx.y * gridDim.x + t);
-  before = __reduce_add_sync(kFull, before);
-  if (lane == 0) s_part[warp] = before;
-  uint32_t id[kRows], in_row[kRows];
-  unsigned right = 0;
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const uint32_t p = blockIdx.x * kTile + r * kThreads + threadIdx.x;
-    id[r] = p < n ? __ldg(list + p) : 0u;
-    const bool one = p < n && side[id[r]] != 0;
-    const unsigned m = __ballot_sync(kFull, one);
-    right |= (one ? 1u : 0u) << r;
-    in_row[r] = __popc(m & lt);
-    if (lane == 0) s_row[r * kWarps + warp] = __popc(m);
-  }
-  __syncthreads();
-  if (warp == 0) {  // exclusive scan of the 64 row pieces, two per lane
-    const uint32_t a = s_row[2 * lane], b = s_row[2 * lane + 1];
-    uint32_t incl = a + b;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(kFull, incl, d);
-      if ((int)lane >= d) incl += t;
+  __device__ void results(uint32_t& swaps, uint32_t& cut) const {
+    const unsigned lane = threadIdx.x & 31u;
+    if (lane == 0) {
+      s.swaps[warp()] = swaps;
+      s.cut[warp()] = cut;
     }
-    s_row[2 * lane] = incl - a - b;
-    s_row[2 * lane + 1] = incl - b;
+    sync();
+    swaps = __reduce_add_sync(kFull, lane < n ? s.swaps[lane] : 0u);
+    cut = __reduce_min_sync(kFull, lane < n ? s.cut[lane] : ~0u);
   }
-  before = 0;
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) before += s_part[w];
-  __syncthreads();
-  const uint32_t q = n >> level;  // the level's range sizes are q and q + 1
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const uint32_t p = blockIdx.x * kTile + r * kThreads + threadIdx.x;
-    if (p >= n) continue;
-    const Range g = range_of(n, level, p);
-    const uint32_t ones = before + s_row[r * kWarps + warp] + in_row[r] - ones_before(g, q);
-    out[(size_t)blockIdx.y * n + ((right >> r) & 1u ? g.m + ones : p - ones)] = id[r];
+};
+
+// The blocks of a cluster.
+struct ClusterTeam {
+  BlockTeam block;
+  unsigned rank;
+  __device__ unsigned warps() const { return block.n * kCluster; }
+  __device__ unsigned warp() const { return rank * block.n + block.warp(); }
+  __device__ void sync() const { cg::this_cluster().sync(); }
+  __device__ const TeamShared& of(unsigned r) const { return *cg::this_cluster().map_shared_rank(&block.s, r); }
+  __device__ void offsets(uint32_t& ge, uint32_t& le) const {
+    block.put_counts(ge, le);
+    const unsigned lane = threadIdx.x & 31u, w = block.warp();
+    const uint32_t g = lane < block.n ? block.s.ge[lane] : 0u, e = lane < block.n ? block.s.le[lane] : 0u;
+    if (w == 0) {
+      const uint32_t all_ge = __reduce_add_sync(kFull, g), all_le = __reduce_add_sync(kFull, e);
+      if (lane == 0) {
+        block.s.all_ge = all_ge;
+        block.s.all_le = all_le;
+      }
+    }
+    sync();
+    ge = __reduce_add_sync(kFull, (lane < w ? g : 0u) + (lane < rank ? of(lane).all_ge : 0u));
+    le = __reduce_add_sync(kFull, (lane > w ? e : 0u) + (lane > rank && lane < kCluster ? of(lane).all_le : 0u));
+  }
+  __device__ void results(uint32_t& swaps, uint32_t& cut) const {
+    block.results(swaps, cut);
+    const unsigned lane = threadIdx.x & 31u;
+    if (threadIdx.x == 0) {
+      block.s.all_swaps = swaps;
+      block.s.all_cut = cut;
+    }
+    sync();
+    swaps = __reduce_add_sync(kFull, lane < kCluster ? of(lane).all_swaps : 0u);
+    cut = __reduce_min_sync(kFull, lane < kCluster ? of(lane).all_cut : ~0u);
+  }
+};
+
+// Partitions a[f, l) (more than three elements) about its pivot and returns the first
+// place of the right part, in (f, l).  Element i has partner number (elements not
+// smaller than the pivot before it) in the left list, or (elements not larger
+// behind it) in the right one; lp, rp: room for (l - f) / 2 places each.
+template <class Team, class Place>
+__device__ __forceinline__ uint32_t partition(const Team& team, Elem* a, uint32_t f, uint32_t l,
+                                              Place* lp, Place* rp) {
+  const unsigned lane = threadIdx.x & 31u, lt = lt_mask();
+  if (team.warp() == 0) {
+    const uint32_t mid = f + (l - f) / 2;
+    const uint32_t at = median_place(f + 1, a[f + 1].key, mid, a[mid].key, l - 1, a[l - 1].key);
+    __syncwarp();
+    if (lane == 0) {
+      const Elem x = a[f];
+      a[f] = a[at];
+      a[at] = x;
+    }
+  }
+  team.sync();
+  const float p = a[f].key;
+  const uint32_t rows = (l - f - 1 + 31) / 32, per = (rows + team.warps() - 1) / team.warps() * 32;
+  const uint32_t b = min(f + 1 + team.warp() * per, l), e = min(b + per, l);
+  uint32_t nge = 0, nle = 0;
+#pragma unroll 4
+  for (uint32_t r = b; r < e; r += 32) {
+    const float k = a[min(r + lane, e - 1)].key;
+    nge += __popc(__ballot_sync(kFull, r + lane < e && !(k < p)));
+    nle += __popc(__ballot_sync(kFull, r + lane < e && !(p < k)));
+  }
+  uint32_t before = nge, behind = nle;
+  team.offsets(before, behind);
+  behind += nle;
+  uint32_t swaps = 0, cut = l;
+#pragma unroll 4
+  for (uint32_t r = b; r < e; r += 32) {
+    const uint32_t i = r + lane;
+    const float k = a[min(i, e - 1)].key;
+    const bool ge = i < e && !(k < p), le = i < e && !(p < k);
+    const unsigned gm = __ballot_sync(kFull, ge), em = __ballot_sync(kFull, le);
+    const uint32_t cg = before + __popc(gm & lt);
+    const uint32_t cl = behind - __popc(em & lt) - (le ? 1u : 0u);
+    const bool left = ge && cl > cg, right = le && cg > cl;
+    if (left) lp[cg] = (Place)i;
+    if (right) rp[cl] = (Place)i;
+    if ((ge && !left) || right) cut = min(cut, i);
+    swaps += __popc(__ballot_sync(kFull, left));
+    before += __popc(gm);
+    behind -= __popc(em);
+  }
+  cut = __reduce_min_sync(kFull, cut);
+  team.results(swaps, cut);
+  for (uint32_t m = team.warp() * 32 + lane; m < swaps; m += team.warps() * 32) {
+    const uint32_t x = lp[m], y = rp[m];
+    const Elem ex = a[x];
+    a[x] = a[y];
+    a[y] = ex;
+  }
+  team.sync();
+  return cut;
+}
+
+// The same of at most 32 elements, lane i holding element i of c; n: the median's
+// place.  Goes on until at most three are left or the partitions are used up;
+// [f, l) is what is left.
+__device__ __forceinline__ void lanes_narrow(Elem& x, uint32_t& f, uint32_t& l, uint32_t nth, int& depth,
+                                             uint8_t* place, unsigned lane) {
+  const unsigned lt = lt_mask();
+  while (l - f > 3 && depth > 0) {
+    --depth;
+    const uint32_t mid = f + (l - f) / 2;
+    const float k1 = __shfl_sync(kFull, x.key, f + 1), k2 = __shfl_sync(kFull, x.key, mid),
+                k3 = __shfl_sync(kFull, x.key, l - 1);
+    const uint32_t at = median_place(f + 1, k1, mid, k2, l - 1, k3);
+    const uint32_t from = lane == f ? at : (lane == at ? f : lane);
+    x.key = __shfl_sync(kFull, x.key, from);
+    x.id = __shfl_sync(kFull, x.id, from);
+    const float p = __shfl_sync(kFull, x.key, f);
+    const bool on = lane > f && lane < l;
+    const bool ge = on && !(x.key < p), le = on && !(p < x.key);
+    const unsigned gm = __ballot_sync(kFull, ge), em = __ballot_sync(kFull, le);
+    const int cg = __popc(gm & lt), cl = __popc(em & ~lt) - (le ? 1 : 0);
+    const bool left = ge && cl > cg, right = le && cg > cl;
+    const unsigned stops = __ballot_sync(kFull, (ge && !left) || right);
+    if (left) place[cg] = (uint8_t)lane;
+    if (right) place[16 + cl] = (uint8_t)lane;
+    __syncwarp();
+    const unsigned partner = left ? place[16 + cg] : (right ? place[cl] : lane);
+    __syncwarp();
+    x.key = __shfl_sync(kFull, x.key, partner);
+    x.id = __shfl_sync(kFull, x.id, partner);
+    const uint32_t cut = stops ? (uint32_t)__ffs(stops) - 1u : l;
+    if (cut <= nth) f = cut;
+    else l = cut;
   }
 }
 
-// The levels below `top` in shared memory: one block per range of at most kRange
-// photons, its three lists as places in its x list.  `inv` (one word per photon)
-// takes the photons' places in that list.  order: the photons of the last level.
-constexpr uint32_t kRange = 1024;
-constexpr int kPer = kRange / kThreads;  // consecutive list places per thread
+// One warp: the selection goes on in a[f, l) with `depth` partitions left.  lp, rp:
+// as for partition(); place: 32 bytes of the warp's own.
+template <class Place>
+__device__ __forceinline__ void warp_select(Elem* a, uint32_t f, uint32_t l, uint32_t nth, int depth,
+                                            Place* lp, Place* rp, uint8_t* place) {
+  const unsigned lane = threadIdx.x & 31u;
+  while (l - f > 32 && depth > 0) {
+    --depth;
+    const uint32_t cut = partition(WarpTeam{}, a, f, l, lp, rp);
+    if (cut <= nth) f = cut;
+    else l = cut;
+  }
+  if (l - f <= 32) {
+    const uint32_t c = l - f, base = f;
+    Elem x = a[base + min(lane, c - 1)];
+    uint32_t lf = 0, ll = c;
+    lanes_narrow(x, lf, ll, nth - base, depth, place, lane);
+    if (ll - lf <= 3) {  // the rest is sorted by insertion, which keeps equal elements' order
+      uint32_t rank = lf;
+      for (uint32_t i = lf; i < ll; ++i) {
+        const float k = __shfl_sync(kFull, x.key, i);
+        rank += k < x.key || (!(x.key < k) && i < lane) ? 1u : 0u;
+      }
+      if (lane < c) a[base + (lane >= lf && lane < ll ? rank : lane)] = x;
+      __syncwarp();
+      return;
+    }
+    if (lane < c) a[base + lane] = x;
+    f = base + lf;
+    l = base + ll;
+    __syncwarp();
+  }
+  if (lane == 0)  // no partitions left: a heap
+    std::__introselect(a + f, a + nth, a + l, 0, __gnu_cxx::__ops::__iter_comp_iter(KeyLess()));
+  __syncwarp();
+}
+
+// Partitions while more than `most` elements are left and partitions are.
+template <class Team, class Place>
+__device__ __forceinline__ void narrow(const Team& team, Elem* a, uint32_t& f, uint32_t& l, uint32_t nth,
+                                       int& depth, uint32_t most, Place* lp, Place* rp) {
+  while (l - f > most && depth > 0) {
+    --depth;
+    const uint32_t cut = partition(team, a, f, l, lp, rp);
+    if (cut <= nth) f = cut;
+    else l = cut;
+  }
+}
+
+// The selection by a team of a block, in shared memory; `refused` is set where a
+// heap over more than kMostHeap elements would have to end it.
+template <class Place>
+__device__ __forceinline__ void team_select(const BlockTeam& team, Elem* a, uint32_t f, uint32_t l,
+                                            uint32_t nth, int depth, Place* lp, Place* rp, uint8_t* place,
+                                            uint32_t* refused) {
+  narrow(team, a, f, l, nth, depth, kWarpRange, lp, rp);
+  if (team.warp() == 0) {
+    if (l - f > kMostHeap) *refused = 1;
+    else warp_select(a, f, l, nth, depth, lp, rp, place);
+  }
+  team.sync();
+}
+
+// ---------------------------------------------------------------------------
+// Levels of ranges larger than kShared: all blocks, over tiles of the ranges, as
+// many of every range as its level's largest has.
+struct Tile {
+  uint32_t range, tile;
+};
+__device__ __forceinline__ Tile tile_of(uint32_t tiles) {
+  return Tile{blockIdx.x / tiles, blockIdx.x % tiles};
+}
+
+// A range's selection between two rounds: what is left of it, the partitions left,
+// and the last round's pivot and result.
+struct PartState {
+  uint32_t f, l;
+  int depth;
+  uint32_t active;  // this round partitions it
+  uint32_t at;      // the pivot's place; it goes to f, and the element of f to `at`
+  Elem pivot, front;
+  uint32_t plain;   // the element at `at` is exchanged with no other
+  uint32_t swaps, cut;
+};
+
+__global__ void __launch_bounds__(kThreads) range_extent(const float* __restrict__ pos,
+                                                         const Elem* __restrict__ w, uint32_t n,
+                                                         int level, uint32_t tiles, uint32_t* ext) {
+  const Tile at = tile_of(tiles);
+  __shared__ Extent s_ext[kWarps];
+  const Range r = range_of(n, level, at.range);
+  const uint32_t b = r.b + at.tile * kTile, e = min(b + kTile, r.e);
+  Extent x = no_extent();
+#pragma unroll 4
+  for (uint32_t i = b + threadIdx.x; i < e; i += kThreads) grow(x, pos, level ? w[i].id : i);
+  warp_extent(x);
+  if ((threadIdx.x & 31u) == 0) s_ext[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    uint32_t v = 0;
+    for (int k = 0; k < kWarps; ++k)
+      v = max(v, threadIdx.x < 3 ? s_ext[k].nlo[threadIdx.x] : s_ext[k].hi[threadIdx.x - 3]);
+    atomicMax(ext + 6 * (size_t)at.range + threadIdx.x, v);
+  }
+}
+__device__ __forceinline__ Extent load_extent(const uint32_t* ext, uint32_t s) {
+  Extent x;
+  for (int a = 0; a < 3; ++a) {
+    x.nlo[a] = __ldg(ext + 6 * (size_t)s + a);
+    x.hi[a] = __ldg(ext + 6 * (size_t)s + 3 + a);
+  }
+  return x;
+}
+
+__global__ void __launch_bounds__(kThreads) load_keys(const float* __restrict__ pos, Elem* w, uint32_t n,
+                                                      int level, uint32_t tiles,
+                                                      const uint32_t* __restrict__ ext) {
+  const Tile at = tile_of(tiles);
+  const Range r = range_of(n, level, at.range);
+  const int axis = widest(load_extent(ext, at.range));
+  const uint32_t b = r.b + at.tile * kTile, e = min(b + kTile, r.e);
+#pragma unroll 4
+  for (uint32_t i = b + threadIdx.x; i < e; i += kThreads) {
+    const uint32_t id = level ? w[i].id : i;
+    w[i] = Elem{split_coord(pos, id, axis), id};
+  }
+}
+
+// One cluster per range.  lp, rp: a range's lists lie at its own place in them.
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kBlock)
+    split_cluster(Elem* w, uint32_t n, int level, uint32_t* lp, uint32_t* rp, uint32_t* refused) {
+  extern __shared__ Elem s_elem[];
+  __shared__ TeamShared s_team;
+  __shared__ uint8_t s_place[32];
+  const unsigned rank = cg::this_cluster().block_rank();
+  const BlockTeam block{kBlock / 32, 0, 0, s_team};
+  const Range r = range_of(n, level, blockIdx.x / kCluster);
+  uint32_t f = r.b, l = r.e;
+  int depth = select_depth(r.e - r.b);
+  narrow(ClusterTeam{block, rank}, w, f, l, r.m, depth, kShared, lp + r.b, rp + r.b);
+  if (rank != 0) return;  // (nothing reads its shared memory any more)
+  if (l - f > kShared) {
+    if (threadIdx.x == 0) *refused = 1;
+    return;
+  }
+  const uint32_t c = l - f;
+  uint16_t* lists = reinterpret_cast<uint16_t*>(s_elem + kShared);
+  for (uint32_t i = threadIdx.x; i < c; i += kBlock) s_elem[i] = w[f + i];
+  __syncthreads();
+  team_select(block, s_elem, 0, c, r.m - f, depth, lists, lists + kShared / 2, s_place, refused);
+  for (uint32_t i = threadIdx.x; i < c; i += kBlock) w[f + i] = s_elem[i];
+}
+
+// ---------------------------------------------------------------------------
+// One block per range of at most `cap` <= kShared photons: one level's split.
+__global__ void __launch_bounds__(kBlock) split_block(const float* __restrict__ pos, Elem* w, uint32_t n,
+                                                      int level, uint32_t cap, uint32_t* refused) {
+  extern __shared__ Elem s_elem[];
+  __shared__ TeamShared s_team;
+  __shared__ uint8_t s_place[32];
+  __shared__ Extent s_ext[kBlock / 32];
+  uint16_t* lists = reinterpret_cast<uint16_t*>(s_elem + cap);
+  const Range r = range_of(n, level, blockIdx.x);
+  const uint32_t c = r.e - r.b;
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  Extent x = no_extent();
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) {
+    const uint32_t id = level ? w[r.b + i].id : i;
+    s_elem[i].id = id;
+    grow(x, pos, id);
+  }
+  warp_extent(x);
+  if (lane == 0) s_ext[warp] = x;
+  __syncthreads();
+  x = lane < (blockDim.x >> 5) ? s_ext[lane] : no_extent();
+  warp_extent(x);
+  const int axis = widest(x);
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) s_elem[i].key = split_coord(pos, s_elem[i].id, axis);
+  __syncthreads();
+  team_select(BlockTeam{blockDim.x >> 5, 0, 0, s_team}, s_elem, 0, c, r.m - r.b, select_depth(c), lists,
+              lists + cap / 2, s_place, refused);
+  for (uint32_t i = threadIdx.x; i < c; i += blockDim.x) w[r.b + i] = s_elem[i];
+}
+
+// One block per range of at most kLeafRange photons: every level below `top`, its
+// warps in as many teams as the level has ranges, or more than one range to a warp.
+// w null: the photons in their own order.  order: the photons of the leaves.
 __global__ void __launch_bounds__(kThreads) split_ranges(const float* __restrict__ pos,
-                                                         const uint32_t* lists, uint32_t* inv,
-                                                         uint32_t n, int top, int depth,
-                                                         uint32_t* order) {
-  __shared__ float s_pos[3][kRange];
-  __shared__ uint32_t s_id[kRange], s_warp[kWarps];
-  __shared__ uint16_t s_list[2][3][kRange];
-  __shared__ uint8_t s_side[kRange];
-  uint32_t b = 0, e = n;
-  for (int l = top - 1; l >= 0; --l) {
-    const uint32_t m = b + (e - b) / 2;
-    if ((blockIdx.x >> l) & 1u) b = m;
-    else e = m;
-  }
-  const uint32_t c = e - b;
+                                                         const Elem* __restrict__ w, uint32_t n, int top,
+                                                         int depth, uint32_t* order, uint32_t* refused) {
+  __shared__ float s_pos[3][kLeafRange];
+  __shared__ uint32_t s_id[kLeafRange];
+  __shared__ Elem s_elem[kLeafRange];
+  __shared__ uint16_t s_lists[kLeafRange];
+  __shared__ TeamShared s_team[kWarps / 2];
+  __shared__ Extent s_ext[kWarps];
+  __shared__ uint8_t s_place[kWarps][32];
+  const Range all = range_of(n, top, blockIdx.x);
+  const uint32_t c = all.e - all.b;
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   for (uint32_t i = threadIdx.x; i < c; i += kThreads) {
-    const uint32_t id = lists[b + i];
+    const uint32_t id = w ? w[all.b + i].id : i;
     s_id[i] = id;
-    inv[id] = i;
-    s_list[0][0][i] = (uint16_t)i;
+    s_elem[i].id = i;
 #pragma unroll
     for (int a = 0; a < 3; ++a) s_pos[a][i] = __ldg(pos + 3 * (size_t)id + a);
   }
   __syncthreads();
-  for (int a = 1; a < 3; ++a)
-    for (uint32_t i = threadIdx.x; i < c; i += kThreads)
-      s_list[0][a][i] = (uint16_t)inv[lists[(size_t)a * n + b + i]];
-  __syncthreads();
-  int cur = 0;
-  for (int level = top; level < depth; ++level, cur ^= 1) {
-    Range g[kPer];
+  for (int level = top; level < depth; ++level) {
+    const uint32_t count = 1u << (level - top);
+    const unsigned tw = count < kWarps ? kWarps / count : 1u;  // warps per team
+    for (uint32_t s = warp / tw; s < count; s += kWarps / tw) {
+      const Range r = range_of(c, level - top, s);
+      const unsigned first = warp / tw * tw, tlane = (warp - first) * 32 + lane;
+      const BlockTeam team{tw, first, 1 + warp / tw, s_team[tw > 1 ? warp / tw : 0]};
+      Extent x = no_extent();
+      for (uint32_t i = r.b + tlane; i < r.e; i += 32 * tw) {
+        const uint32_t j = s_elem[i].id;
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const uint32_t p = kPer * threadIdx.x + j;
-      if (p >= c) continue;
-      g[j] = range_of(c, level - top, p);
-      float ext[3];
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        ext[a] = s_pos[a][s_list[cur][a][g[j].e - 1]] - s_pos[a][s_list[cur][a][g[j].b]];
-      int axis = 0;
-      if (ext[1] > ext[0]) axis = 1;
-      if (ext[2] > (axis == 1 ? ext[1] : ext[0])) axis = 2;
-      s_side[s_list[cur][axis][p]] = p >= g[j].m ? 1 : 0;
-    }
-    __syncthreads();
-    const uint32_t q = c >> (level - top);
-    const int nlists = level == depth - 1 ? 1 : 3;
-    for (int a = 0; a < nlists; ++a) {
-      uint32_t id[kPer], one[kPer], sum = 0, total;
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        const uint32_t p = kPer * threadIdx.x + j;
-        id[j] = p < c ? s_list[cur][a][p] : 0u;
-        one[j] = p < c ? s_side[id[j]] : 0u;
-        sum += one[j];
+        for (int a = 0; a < 3; ++a) grow(x, a, s_pos[a][j]);
       }
-      uint32_t before = block_scan(sum, s_warp, &total);
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        const uint32_t p = kPer * threadIdx.x + j;
-        if (p < c) {
-          const uint32_t ones = before - ones_before(g[j], q);
-          s_list[cur ^ 1][a][one[j] ? g[j].m + ones : p - ones] = (uint16_t)id[j];
-        }
-        before += one[j];
+      warp_extent(x);
+      if (tw > 1) {
+        if (lane == 0) s_ext[warp] = x;
+        team.sync();
+        x = lane < tw ? s_ext[first + lane] : no_extent();
+        warp_extent(x);
+      }
+      const int axis = widest(x);
+      for (uint32_t i = r.b + tlane; i < r.e; i += 32 * tw) {
+        const float v = s_pos[axis][s_elem[i].id];
+        s_elem[i].key = isnan(v) ? INFINITY : v;
+      }
+      uint16_t *lp = s_lists + r.b, *rp = lp + (r.e - r.b) / 2;
+      if (tw > 1) {
+        team.sync();
+        team_select(team, s_elem, r.b, r.e, r.m, select_depth(r.e - r.b), lp, rp, s_place[warp], refused);
+      } else {
+        __syncwarp();
+        warp_select(s_elem, r.b, r.e, r.m, select_depth(r.e - r.b), lp, rp, s_place[warp]);
       }
     }
     __syncthreads();
   }
-  for (uint32_t i = threadIdx.x; i < c; i += kThreads) order[b + i] = s_id[s_list[cur][0][i]];
+  for (uint32_t i = threadIdx.x; i < c; i += kThreads) order[all.b + i] = s_id[s_elem[i].id];
 }
 
 // The bounds of a warp's 32 boxes to item j of a level's arrays.
@@ -394,9 +623,7 @@ __device__ __forceinline__ void put_bounds(float (&lo)[3], float (&hi)[3], float
 }
 
 // One warp per leaf (pad of them; those past count get inverted boxes): its
-// range, its photons' records and their bounds.  The photons lie in a stride
-// through their x order: a leaf in x order offers a gather's heap ever nearer
-// photons, each of which replaces the maximum (2.7 % on a k = 50 gather).
+// range, its photons' records and their bounds.
 __global__ void __launch_bounds__(kThreads) write_leaves(
     const float* __restrict__ pos, const float* __restrict__ nrm, const float* __restrict__ pw,
     const uint32_t* __restrict__ order, uint32_t n, int depth, uint32_t count, uint32_t pad,
@@ -415,9 +642,7 @@ __global__ void __launch_bounds__(kThreads) write_leaves(
     if (lane == 0) leaf[j] = make_uint2(b, e);
     const uint32_t c = e - b;  // at most 32
     if (lane < c) {
-      const uint32_t stride = c % 11u ? 11u : 13u;  // coprime to c
-      const uint32_t i = b + (lane * stride) % c;
-      const uint32_t s = order ? __ldg(order + i) : i;
+      const uint32_t s = order ? __ldg(order + b + lane) : b + lane;
       const size_t k = 3 * (size_t)s;
       const float4 p = make_float4(__ldg(pos + k), __ldg(pos + k + 1), __ldg(pos + k + 2),
                                    __int_as_float((int)s));
@@ -453,50 +678,62 @@ __global__ void __launch_bounds__(kThreads) write_boxes(float* box, uint32_t cou
 
 }  // namespace
 
+namespace {
+
+size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+uint32_t most_in_range(size_t n, int level) {
+  return (uint32_t)((n + ((size_t)1 << level) - 1) >> level);
+}
+// Ranges of the last level that split_cluster splits.
+size_t cluster_ranges(size_t n) {
+  int level = 0;
+  while (most_in_range(n, level) > kShared) ++level;
+  return (size_t)1 << (level > 0 ? level - 1 : 0);
+}
+
+}  // namespace
+
 size_t photon_build_scratch(size_t n) {
-  const size_t tiles = (n + kTile - 1) / kTile;
-  return 4 * n + 256 + n + 256 + (3 * 256 * tiles + 3 * 256) * 4;
+  return up256(4 * n) + up256(24 * cluster_ranges(n)) + 256;
 }
 
 int build_photon_device(const float* pos, const float* nrm, const float* pw, const DevPhotonMap& d,
-                        void* scratch) {
+                        void* scratch, bool* refused) {
   const uint32_t n = d.n;
-  const size_t tiles = (n + kTile - 1) / kTile;
-  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-  // The record arrays, written last, hold the items while they are sorted (24
-  // bytes per photon each, in turn) and then, in their second half, the lists
-  // (12 each, in turn); the last level's x list, the order of the records, and
-  // the counts lie in the scratch.
-  uint2* items[2] = {reinterpret_cast<uint2*>(d.d_pos4),
-                     reinterpret_cast<uint2*>(d.d_pos4) + 3 * (size_t)n};
-  uint32_t* lists[2] = {reinterpret_cast<uint32_t*>(items[1]),
-                        reinterpret_cast<uint32_t*>(items[1]) + 3 * (size_t)n};
+  const size_t ranges = cluster_ranges(n);
+  // The record arrays, written last, hold the elements and the lists of the
+  // partitions (8, 4 and 4 bytes per photon); the order of the records and the
+  // tables lie in the scratch.
+  Elem* w = reinterpret_cast<Elem*>(d.d_pos4);
+  uint32_t* lp = reinterpret_cast<uint32_t*>(w + n);
+  uint32_t* rp = lp + n;
   char* base = static_cast<char*>(scratch);
   uint32_t* order = reinterpret_cast<uint32_t*>(base);
-  uint8_t* side = reinterpret_cast<uint8_t*>(base + up(4 * (size_t)n));
-  uint32_t* hist = reinterpret_cast<uint32_t*>(base + up(4 * (size_t)n) + up(n));
-  uint32_t* sums = hist + 3 * 256 * tiles;
-  const dim3 tg((unsigned)tiles, 3);
-  const unsigned flat =
-      (unsigned)std::min<size_t>(((size_t)n + kThreads - 1) / kThreads, (size_t)device_sm_count(d.device) * 8);
+  base += up256(4 * (size_t)n);
+  uint32_t* ext = reinterpret_cast<uint32_t*>(base);
+  uint32_t* flag = reinterpret_cast<uint32_t*>(base + up256(24 * ranges));
+  cudaError_t e = cudaMemsetAsync(flag, 0, 4);
+  const size_t full = kShared * kElemBytes;
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(split_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)full);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(split_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)full);
+  if (e != cudaSuccess) return (int)e;
   if (d.depth > 0) {
-    static_assert(kPasses % 2 == 0, "the last pass reads items[0] and writes over items[1]");
-    for (int pass = 0; pass < kPasses; ++pass) {
-      const uint2* in = pass == 0 ? nullptr : items[(pass & 1) ^ 1];
-      sort_count<<<tg, kThreads>>>(pos, in, n, pass, hist);
-      sort_scan<<<dim3(256, 3), kThreads>>>(hist, (uint32_t)tiles, sums);
-      sort_move<<<tg, kThreads>>>(pos, in, n, pass, hist, sums, items[pass & 1],
-                                  pass == kPasses - 1 ? lists[0] : nullptr);
+    int level = 0;
+    for (; most_in_range(n, level) > kShared; ++level) {
+      const uint32_t c = most_in_range(n, level), count = 1u << level;
+      const uint32_t tiles = (c + kTile - 1) / kTile, grid = tiles * count;
+      if ((e = cudaMemsetAsync(ext, 0, 24 * (size_t)count)) != cudaSuccess) return (int)e;
+      range_extent<<<grid, kThreads>>>(pos, w, n, level, tiles, ext);
+      load_keys<<<grid, kThreads>>>(pos, w, n, level, tiles, ext);
+      split_cluster<<<count * kCluster, kBlock, full>>>(w, n, level, lp, rp, flag);
     }
-    int cur = 0, top = 0;
-    while (((n + (1ull << top) - 1) >> top) > kRange) {
-      split_side<<<flat, kThreads>>>(pos, lists[cur], n, top, side);
-      split_count<<<tg, kThreads>>>(lists[cur], side, n, hist);
-      split_move<<<tg, kThreads>>>(lists[cur], side, n, top, hist, lists[cur ^ 1]);
-      cur ^= 1;
-      ++top;
+    for (; level < d.depth && most_in_range(n, level) > kLeafRange; ++level) {
+      const uint32_t cap = (most_in_range(n, level) + 1) / 2 * 2;
+      split_block<<<1u << level, kBlock, cap * kElemBytes>>>(pos, w, n, level, cap, flag);
     }
-    split_ranges<<<1u << top, kThreads>>>(pos, lists[cur], lists[cur ^ 1], n, top, d.depth, order);
+    split_ranges<<<1u << level, kThreads>>>(pos, level ? w : nullptr, n, level, d.depth, order, flag);
   }
   write_leaves<<<(d.lvl_pad[0] + kWarps - 1) / kWarps, kThreads>>>(
       pos, nrm, pw, d.depth > 0 ? order : nullptr, n, d.depth, d.lvl_count[0], d.lvl_pad[0],
@@ -507,8 +744,12 @@ int build_photon_device(const float* pos, const float* nrm, const float* pw, con
     write_boxes<<<(d.lvl_pad[l] + kWarps - 1) / kWarps, kThreads>>>(
         d.d_box + d.lvl_off[l], d.lvl_count[l], d.lvl_pad[l], d.d_box + d.lvl_off[l - 1],
         d.lvl_count[l - 1], d.lvl_pad[l - 1]);
-  const cudaError_t e = cudaGetLastError();
-  return e != cudaSuccess ? (int)e : (int)cudaStreamSynchronize(0);
+  e = cudaGetLastError();
+  uint32_t bad = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, flag, 4, cudaMemcpyDeviceToHost, 0);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  *refused = bad != 0;
+  return (int)e;
 }
 
 }  // namespace enc
