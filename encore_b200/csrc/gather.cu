@@ -99,11 +99,13 @@ constexpr uint32_t kCountBits = 63u;
 // searched between 0 and the largest: on a surface the number of photons within
 // a distance grows with its square, so interpolating the counts finds one in a
 // few steps; after kGuesses of them the interval is halved, and entries of equal
-// distance at its end are kept in order.  Squared distances are non-negative, so
-// their bit patterns order as unsigned integers.
+// distance at its end are kept in order; *tie is that distance then (some of its
+// entries were dropped).  Squared distances are non-negative, so their bit
+// patterns order as unsigned integers.
 constexpr int kGuesses = 8;
 template <int S>
-__device__ __forceinline__ float keep_nearest(uint2* buf, int count, int k, int lane, unsigned lt) {
+__device__ __forceinline__ float keep_nearest(uint2* buf, int count, int k, int lane, unsigned lt,
+                                              uint32_t* tie) {
   uint2 e[S];
   uint32_t top = 0;
 #pragma unroll
@@ -117,6 +119,7 @@ __device__ __forceinline__ float keep_nearest(uint2* buf, int count, int k, int 
   for (int i = 0;; ++i) {
     if (hi - lo == 1) {
       ties = k - clo;
+      if (lane == 0) *tie = lo;
       break;
     }
     uint32_t t = lo + (hi - lo) / 2;
@@ -178,23 +181,232 @@ __device__ __forceinline__ void sort_entries(uint2* buf, int count, int n, int l
     }
 }
 
+// Which of several photons at the k-th distance are kept.  Until a query holds k
+// photons it takes what it accepts; from then on a nearer photon replaces the
+// farthest one held, of equally far ones the one in the highest slot.  The photons
+// of one step come in the order of their lanes.  The buffer's selection gives the
+// same set unless it drops some of the photons at the k-th distance; such a query
+// (one in some 600,000 of a room's) is walked once more with these slots.  The
+// photons at the k-th distance that the first walk does not accept come after
+// those it does, so neither walk takes them.
+__device__ __forceinline__ int heap_insert(uint2* buf, int count, int k, unsigned m, float d2,
+                                           unsigned pidx, float& r2, int lane, unsigned lt) {
+  auto farthest = [&](uint32_t& far) {  // its slot
+    uint32_t v = 0;
+    int at = -1;
+    for (int i = lane; i < k; i += 32)
+      if (at < 0 || buf[i].x >= v) {
+        v = buf[i].x;
+        at = i;
+      }
+    far = __reduce_max_sync(kFull, v);
+    return (int)__reduce_max_sync(kFull, at >= 0 && v == far ? (uint32_t)at : 0u);
+  };
+  uint32_t far = 0;
+  int slot = 0;
+  const int rank = __popc(m & lt), fill = min(__popc(m), k - count);
+  if (fill > 0) {
+    if (((m >> lane) & 1u) && rank < fill) buf[count + rank] = make_uint2(__float_as_uint(d2), pidx);
+    __syncwarp();
+    count += fill;
+    for (int i = 0; i < fill; ++i) m &= m - 1u;
+    if (count < k) return count;
+  } else if (m == 0) {
+    return count;
+  }
+  slot = farthest(far);
+  for (; m; m &= m - 1u) {
+    const int j = __ffs(m) - 1;
+    const uint32_t d = __float_as_uint(__shfl_sync(kFull, d2, j));
+    const unsigned p = __shfl_sync(kFull, pidx, j);
+    if (d >= far) continue;
+    __syncwarp();
+    if (lane == 0) buf[slot] = make_uint2(d, p);
+    __syncwarp();
+    slot = farthest(far);
+  }
+  __syncwarp();
+  r2 = __uint_as_float(far);
+  return count;
+}
+
+// What COUNT records per query: child boxes and photons tested, normals read.
+struct Work {
+  uint32_t box = 0, pos = 0, nrm = 0;
+};
+struct Query {
+  float x, y, z, nx, ny, nz;
+};
+__device__ __forceinline__ Query load_query(const GatherParams& P, unsigned q) {
+  const float *p = P.qpos + 3 * (size_t)q, *n = P.qnrm + 3 * (size_t)q;
+  return Query{__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(n), __ldg(n + 1), __ldg(n + 2)};
+}
+
+// Walks the tree for one query.  HEAP false: accepted photons go to the buffer, of
+// which the k nearest are kept; r2: the search radius, at the end the k-th distance
+// if any selection was made.  HEAP true: at most k are held, and an accepted photon
+// that finds them full takes the place of the farthest (heap_walk).  Returns the
+// photons held, in buf.
+template <int S, bool HEAP, bool COUNT>
+__device__ __forceinline__ int walk(const GatherParams& P, const Query& q, float& r2, uint2* buf,
+                                    uint2* stk, int lane, unsigned lt, uint32_t* tie, Work& work) {
+  const int k = P.k, depth = 32 * P.nlevels;  // stack entries of a warp
+  const float qx = q.x, qy = q.y, qz = q.z, nx = q.nx, ny = q.ny, nz = q.nz;
+  int count = 0;
+  // the root: the top level's items are its children
+  int sp = 0;
+  if (k > 0) {
+    if (lane == 0) stk[0] = make_uint2((uint32_t)P.nlevels << 28, 0u);
+    sp = 1;
+  }
+  __syncwarp();
+  unsigned steps = 0;
+  while (sp > 0) {
+    if (++steps > kMaxSteps) {
+      if (lane == 0) atomicOr(P.status, 1u);
+      break;
+    }
+    --sp;
+    const uint2 top = stk[sp];
+    const uint32_t e = top.x;
+    if (!(__uint_as_float(top.y & ~kCountBits) < r2)) {  // nothing in it can be accepted
+      __syncwarp();
+      continue;
+    }
+    if (!(e & kLeafEntry)) {
+      __syncwarp();
+      // inner node: lane c tests child 32 * it + c of level lv - 1
+      const int cl = (int)(e >> 28) - 1;
+      const uint32_t child = 32u * (e & 0x0fffffffu) + (uint32_t)lane;
+      bool pass = false;
+      float cd = 0.f;
+      if (child < P.lvl_count[cl]) {
+        const float* b = P.box + P.lvl_off[cl];
+        const uint32_t pad = P.lvl_pad[cl];
+        const float lx = __ldg(b + child), ly = __ldg(b + pad + child),
+                    lz = __ldg(b + 2 * pad + child);
+        const float hx = __ldg(b + 3 * pad + child), hy = __ldg(b + 4 * pad + child),
+                    hz = __ldg(b + 5 * pad + child);
+        const float gx = fmaxf(fmaxf(fs(lx, qx), fs(qx, hx)), 0.f);
+        const float gy = fmaxf(fmaxf(fs(ly, qy), fs(qy, hy)), 0.f);
+        const float gz = fmaxf(fmaxf(fs(lz, qz), fs(qz, hz)), 0.f);
+        cd = fa(fa(fm(gx, gx), fm(gy, gy)), fm(gz, gz));
+        pass = cd < r2;
+      }
+      const unsigned m = __ballot_sync(kFull, pass);
+      if (COUNT) work.box += __popc(__ballot_sync(kFull, child < P.lvl_count[cl]));
+      const int n = __popc(m);
+      if (sp + n > depth) {
+        if (lane == 0) atomicOr(P.status, 2u);
+        break;
+      }
+      // Nearest child on top: the passing children are pushed farthest
+      // first, so the walk visits them nearest first, the buffer fills with
+      // nearer photons and the search radius, once k are kept,
+      // shrinks sooner.  A child's place = the passing children farther
+      // than it (equal distances: the higher lane counts as farther).
+      int farther = 0;
+      for (unsigned mm = m; mm; mm &= mm - 1u) {
+        const int j = __ffs(mm) - 1;
+        const float dj = __shfl_sync(kFull, cd, j);
+        farther += (dj > cd || (dj == cd && j > (int)lane)) ? 1 : 0;
+      }
+      if (pass) {
+        const int at = sp + farther;
+        uint32_t item = ((uint32_t)cl << 28) | child;
+        uint32_t cnt = 0;
+        if (cl == 0) {  // a leaf: its photon range goes onto the stack
+          const uint2 rng = __ldg(P.leaf + child);
+          item = kLeafEntry | rng.x;
+          cnt = rng.y - rng.x;
+        }
+        stk[at] = make_uint2(item, (__float_as_uint(cd) & ~kCountBits) | cnt);
+      }
+      sp += n;
+      __syncwarp();
+      continue;
+    }
+    // leaf: lane j tests photon j of the leaf; when the entry below is a
+    // leaf too and both fit in the warp, lanes c0.. test its photons
+    const int c0 = (int)(top.y & kCountBits);
+    uint32_t b1 = 0;
+    int c1 = 0;
+    if (sp > 0) {
+      const uint2 next = stk[sp - 1];
+      const int n1 = (int)(next.y & kCountBits);
+      if ((next.x & kLeafEntry) && c0 + n1 <= 32 &&
+          __uint_as_float(next.y & ~kCountBits) < r2) {
+        b1 = next.x & ~kLeafEntry;
+        c1 = n1;
+        --sp;
+      }
+    }
+    __syncwarp();
+    const unsigned pidx = lane < c0 ? (e & ~kLeafEntry) + (unsigned)lane
+                                    : b1 + (unsigned)(lane - c0);
+    bool acc = false;
+    float d2 = 0.f;
+    if (COUNT) {
+      work.pos += (uint32_t)(c0 + c1);
+    }
+    if (lane < c0 + c1) {
+      const float4 p = __ldg(P.pos4 + pidx);
+      const float x = fs(qx, p.x), y = fs(qy, p.y), z = fs(qz, p.z);
+      d2 = fa(fa(fm(x, x), fm(y, y)), fm(z, z));
+      acc = d2 < r2;
+      if (acc && !P.ignore_normal) {
+        const float4 pn = __ldg(P.nrm4 + pidx);
+        acc = (pn.x == nx) && (pn.y == ny) && (pn.z == nz);
+      }
+    }
+    if (COUNT && !P.ignore_normal)
+      work.nrm += __popc(__ballot_sync(kFull, lane < c0 + c1 && d2 < r2));
+    const unsigned m = __ballot_sync(kFull, acc);
+    if (HEAP) {
+      count = heap_insert(buf, count, k, m, d2, pidx, r2, lane, lt);
+      continue;
+    }
+    if (acc) buf[count + __popc(m & lt)] = make_uint2(__float_as_uint(d2), pidx);
+    count += __popc(m);
+    __syncwarp();
+    if (count > P.full) {
+      r2 = keep_nearest<S>(buf, count, k, lane, lt, tie);
+      count = k;
+    }
+  }
+  if (!HEAP && count > k) {
+    r2 = keep_nearest<S>(buf, count, k, lane, lt, tie);
+    count = k;
+  }
+  return count;
+}
+
+// Rare, and kept out of the kernel's own code and registers.
+__device__ __noinline__ int heap_walk(const GatherParams& P, unsigned index, uint2* buf, uint2* stk) {
+  const int lane = threadIdx.x & 31;
+  const Query q = load_query(P, index);
+  float r2 = P.r2max;
+  Work work;
+  return walk<1, true, false>(P, q, r2, buf, stk, lane, (1u << lane) - 1u, nullptr, work);
+}
+
 // COUNT: also records per query the work behind the roofline's bytes:
 // visits[4q] child boxes tested (24 bytes each), [4q+1] photons tested (a
 // 16-byte position each), [4q+2] normals read (16 bytes each), [4q+3]
 // photons found (their 16-byte power is read by the estimate).
 template <int S, bool NEAREST, bool COUNT = false>
-__global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
+__global__ void __launch_bounds__(256) gather_kernel(const __grid_constant__ GatherParams P) {
   constexpr int kCap = 32 * S;  // candidates a warp holds: k <= kCap - 32
   // per warp: candidates; stack entries, their squared distances, and a leaf
   // entry's photon count
   __shared__ uint2 s_buf[kWarpsPerBlock][kCap];
+  __shared__ uint32_t s_tie[kWarpsPerBlock];  // the distance of photons dropped at the k-th place
   extern __shared__ uint2 s_dyn[];
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const int k = P.k;
-  const int depth = 32 * P.nlevels;  // stack entries of a warp
-  uint2* stk = s_dyn + wib * depth;
+  uint2* stk = s_dyn + wib * 32 * P.nlevels;
   uint2* buf = s_buf[wib];
   // Each warp takes P.chunk queries at a time from the launch's queue head, so
   // every warp stays busy until the queue is empty (a fixed share per warp left
@@ -214,134 +426,14 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
       q = b;
       qend = min(b + max(P.chunk, 1u), P.nq);
     }
-    const float qx = __ldg(P.qpos + 3 * (size_t)q), qy = __ldg(P.qpos + 3 * (size_t)q + 1),
-                qz = __ldg(P.qpos + 3 * (size_t)q + 2);
-    const float nx = __ldg(P.qnrm + 3 * (size_t)q), ny = __ldg(P.qnrm + 3 * (size_t)q + 1),
-                nz = __ldg(P.qnrm + 3 * (size_t)q + 2);
-    int count = 0;
+    const Query query = load_query(P, q);
+    if (lane == 0) s_tie[wib] = ~0u;
     float r2 = P.r2max;
-    // the root: the top level's items are its children
-    int sp = 0;
-    if (k > 0) {
-      if (lane == 0) stk[0] = make_uint2((uint32_t)P.nlevels << 28, 0u);
-      sp = 1;
-    }
+    Work work;
+    int count = walk<S, false, COUNT>(P, query, r2, buf, stk, lane, lt, &s_tie[wib], work);
     __syncwarp();
-    unsigned steps = 0;
-    uint32_t n_box = 0, n_pos = 0, n_nrm = 0;
-    while (sp > 0) {
-      if (++steps > kMaxSteps) {
-        if (lane == 0) atomicOr(P.status, 1u);
-        break;
-      }
-      --sp;
-      const uint2 top = stk[sp];
-      const uint32_t e = top.x;
-      if (!(__uint_as_float(top.y & ~kCountBits) < r2)) {  // nothing in it can be accepted
-        __syncwarp();
-        continue;
-      }
-      if (!(e & kLeafEntry)) {
-        __syncwarp();
-        // inner node: lane c tests child 32 * it + c of level lv - 1
-        const int cl = (int)(e >> 28) - 1;
-        const uint32_t child = 32u * (e & 0x0fffffffu) + (uint32_t)lane;
-        bool pass = false;
-        float cd = 0.f;
-        if (child < P.lvl_count[cl]) {
-          const float* b = P.box + P.lvl_off[cl];
-          const uint32_t pad = P.lvl_pad[cl];
-          const float lx = __ldg(b + child), ly = __ldg(b + pad + child),
-                      lz = __ldg(b + 2 * pad + child);
-          const float hx = __ldg(b + 3 * pad + child), hy = __ldg(b + 4 * pad + child),
-                      hz = __ldg(b + 5 * pad + child);
-          const float gx = fmaxf(fmaxf(fs(lx, qx), fs(qx, hx)), 0.f);
-          const float gy = fmaxf(fmaxf(fs(ly, qy), fs(qy, hy)), 0.f);
-          const float gz = fmaxf(fmaxf(fs(lz, qz), fs(qz, hz)), 0.f);
-          cd = fa(fa(fm(gx, gx), fm(gy, gy)), fm(gz, gz));
-          pass = cd < r2;
-        }
-        const unsigned m = __ballot_sync(kFull, pass);
-        if (COUNT) n_box += __popc(__ballot_sync(kFull, child < P.lvl_count[cl]));
-        const int n = __popc(m);
-        if (sp + n > depth) {
-          if (lane == 0) atomicOr(P.status, 2u);
-          break;
-        }
-        // Nearest child on top: the passing children are pushed farthest
-        // first, so the walk visits them nearest first, the buffer fills with
-        // nearer photons and the search radius, once k are kept,
-        // shrinks sooner.  A child's place = the passing children farther
-        // than it (equal distances: the higher lane counts as farther).
-        int farther = 0;
-        for (unsigned mm = m; mm; mm &= mm - 1u) {
-          const int j = __ffs(mm) - 1;
-          const float dj = __shfl_sync(kFull, cd, j);
-          farther += (dj > cd || (dj == cd && j > (int)lane)) ? 1 : 0;
-        }
-        if (pass) {
-          const int at = sp + farther;
-          uint32_t item = ((uint32_t)cl << 28) | child;
-          uint32_t cnt = 0;
-          if (cl == 0) {  // a leaf: its photon range goes onto the stack
-            const uint2 rng = __ldg(P.leaf + child);
-            item = kLeafEntry | rng.x;
-            cnt = rng.y - rng.x;
-          }
-          stk[at] = make_uint2(item, (__float_as_uint(cd) & ~kCountBits) | cnt);
-        }
-        sp += n;
-        __syncwarp();
-        continue;
-      }
-      // leaf: lane j tests photon j of the leaf; when the entry below is a
-      // leaf too and both fit in the warp, lanes c0.. test its photons
-      const int c0 = (int)(top.y & kCountBits);
-      uint32_t b1 = 0;
-      int c1 = 0;
-      if (sp > 0) {
-        const uint2 next = stk[sp - 1];
-        const int n1 = (int)(next.y & kCountBits);
-        if ((next.x & kLeafEntry) && c0 + n1 <= 32 &&
-            __uint_as_float(next.y & ~kCountBits) < r2) {
-          b1 = next.x & ~kLeafEntry;
-          c1 = n1;
-          --sp;
-        }
-      }
-      __syncwarp();
-      const unsigned pidx = lane < c0 ? (e & ~kLeafEntry) + (unsigned)lane
-                                      : b1 + (unsigned)(lane - c0);
-      bool acc = false;
-      float d2 = 0.f;
-      if (COUNT) {
-        n_pos += (uint32_t)(c0 + c1);
-      }
-      if (lane < c0 + c1) {
-        const float4 p = __ldg(P.pos4 + pidx);
-        const float x = fs(qx, p.x), y = fs(qy, p.y), z = fs(qz, p.z);
-        d2 = fa(fa(fm(x, x), fm(y, y)), fm(z, z));
-        acc = d2 < r2;
-        if (acc && !P.ignore_normal) {
-          const float4 pn = __ldg(P.nrm4 + pidx);
-          acc = (pn.x == nx) && (pn.y == ny) && (pn.z == nz);
-        }
-      }
-      if (COUNT && !P.ignore_normal)
-        n_nrm += __popc(__ballot_sync(kFull, lane < c0 + c1 && d2 < r2));
-      const unsigned m = __ballot_sync(kFull, acc);
-      if (acc) buf[count + __popc(m & lt)] = make_uint2(__float_as_uint(d2), pidx);
-      count += __popc(m);
-      __syncwarp();
-      if (count > P.full) {
-        r2 = keep_nearest<S>(buf, count, k, lane, lt);
-        count = k;
-      }
-    }
-    if (count > k) {
-      keep_nearest<S>(buf, count, k, lane, lt);
-      count = k;
-    }
+    if (count == k && s_tie[wib] == __float_as_uint(r2)) count = heap_walk(P, q, buf, stk);
+    __syncwarp();
 
     if (NEAREST) {
       // by distance, then by the photon's index
@@ -396,9 +488,9 @@ __global__ void __launch_bounds__(256) gather_kernel(GatherParams P) {
       __syncwarp();
     }
     if (COUNT && lane == 0) {
-      P.visits[4 * (size_t)q] = n_box;
-      P.visits[4 * (size_t)q + 1] = n_pos;
-      P.visits[4 * (size_t)q + 2] = n_nrm;
+      P.visits[4 * (size_t)q] = work.box;
+      P.visits[4 * (size_t)q + 1] = work.pos;
+      P.visits[4 * (size_t)q + 2] = work.nrm;
       P.visits[4 * (size_t)q + 3] = (uint32_t)count;
     }
     ++q;
