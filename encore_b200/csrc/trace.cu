@@ -1321,6 +1321,7 @@ __global__ void __launch_bounds__(128, kKdBlocks) kd_trace(KdParams P) {
         cnt = 0;
         if (!in) node = kNoItem;  // no walk: ends below as a miss
       }
+      __syncwarp();  // the other lanes read a fresh ray and write its hit (a ballot orders no memory)
     }
     if (__ballot_sync(kFull, active) == 0) break;
 
