@@ -1574,6 +1574,14 @@ bool many_rays(size_t n, int blocks, int threads) {
   return n >= (size_t)blocks * (size_t)threads * 6;
 }
 
+// A launch gets 48 KB of shared memory per block without asking for more, and the
+// traversal's own arrays (9.2 KB) are part of it beside the stacks.
+template <class Kernel>
+cudaError_t allow_shared(Kernel k, size_t stacks) {
+  if (stacks <= 36 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stacks);
+}
+
 template <bool CLAMP, bool ANY>
 int launch_few(TraceParams p, size_t n, int sms, cudaStream_t s) {
   const size_t warps = (size_t)sms * kSpreadWarps;
@@ -1633,10 +1641,7 @@ int launch_w(const DevAccel& a, const float* rays, size_t n, void* out, uint32_t
       }
     }
   }
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  if (const cudaError_t e = allow_shared(k, smem); e != cudaSuccess) return (int)e;
   int grid = sms * (L.blocks_per_sm > 0
                         ? L.blocks_per_sm
                         : (ANY ? kBlocksAny : (lane ? kBlocksLane : kBlocksClosest)));
@@ -1760,10 +1765,7 @@ int launch_w_external(const DevAccel& a, const float* rays, size_t n, enc_hit* h
   }
   size_t smem = (size_t)p.stack_depth * L.block * stack_entry_bytes(W);
   auto k = wbvh_trace<W, CLAMP, false, false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  if (const cudaError_t e = allow_shared(k, smem); e != cudaSuccess) return (int)e;
   int grid = sms * (L.blocks_per_sm > 0 ? L.blocks_per_sm : kBlocksClosest);
   if (n > 0) p.share = ray_share(L, n, sms, &grid);
   k<<<grid, L.block, smem, s>>>(p);
@@ -1843,10 +1845,7 @@ int launch_multi_w(const MultiLaunch& m, const Launch& L, cudaStream_t s) {
     if (m.wait && many_rays(m.total, blocks, L.block))
       k = wbvh_trace<W, CLAMP, false, false, true, false, false, true>;
   }
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  if (const cudaError_t e = allow_shared(k, smem); e != cudaSuccess) return (int)e;
   cudaError_t e = cudaMemsetAsync(m.d_counter, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return (int)e;
   int grid = device_sm_count(m.device) *
