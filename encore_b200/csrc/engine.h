@@ -3,6 +3,7 @@
 // structure and the kernel that walks it agree by construction.
 #pragma once
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <mutex>
@@ -212,6 +213,29 @@ struct Launch {
   bool per_lane = false;
 };
 Launch resolve_launch(const enc_launch_opts* o, int kind, int width);
+
+// Warps per SM that a batch smaller than one grid of 32-ray chunks is spread
+// over.  Such a launch lasts as long as its slowest warp, and a warp with
+// fewer rays steps faster (fewer triangle rounds, fewer divergent refills),
+// while more warps slow one another down.  With wbvh_trace (at width 8 wbvh_few
+// takes up to 28,416 rays), 777 eye rays on 10,000 triangles took
+// 76 us with 32 rays per warp on every resident warp's queue, 49 us at 16;
+// 20,000 rays: 104 us, and 84 / 80 / 88 / 106 us at 8 / 12 / 16 / 36; 100,000
+// rays: 153 us, 117 us at 8 to 16 (32 rays per warp, fewer blocks).
+constexpr int kSpreadWarps = 16;
+
+// The share of each warp of a launch over n rays on at most *grid blocks (the
+// caller's choice of blocks per SM among them), and the blocks that cover them; 0
+// where the warps take their rays through the queue: the batch exceeds one chunk
+// per warp of the grid, or the caller chose the chunk.
+inline unsigned ray_share(const Launch& L, size_t n, int sms, int* grid) {
+  const size_t wpb = (size_t)L.block / 32, warps = (size_t)*grid * wpb;
+  if (L.fixed_chunk || n > warps * 32) return 0;
+  const size_t want = std::min((size_t)sms * kSpreadWarps, warps);
+  const size_t share = std::clamp<size_t>((n + want - 1) / want, 1, 32);
+  *grid = (int)std::max<size_t>(1, (n + share * wpb - 1) / (share * wpb));
+  return (unsigned)share;
+}
 
 // ---------------------------------------------------------------------------
 // Ray binning (reorder.cu): a key per ray from its origin cell and direction

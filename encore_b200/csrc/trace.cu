@@ -1522,29 +1522,6 @@ constexpr size_t stack_entry_bytes(int W) {
   return W == 8 ? sizeof(uint2) : sizeof(uint2) + sizeof(float);
 }
 
-// Warps per SM that a batch smaller than one grid of 32-ray chunks is spread
-// over.  Such a launch lasts as long as its slowest warp, and a warp with
-// fewer rays steps faster (fewer triangle rounds, fewer divergent refills),
-// while more warps slow one another down.  With this kernel (width 8 hands up to
-// 28,416 rays to wbvh_few, below), 777 eye rays on 10,000 triangles took
-// 76 us with 32 rays per warp on every resident warp's queue, 49 us at 16;
-// 20,000 rays: 104 us, and 84 / 80 / 88 / 106 us at 8 / 12 / 16 / 36; 100,000
-// rays: 153 us, 117 us at 8 to 16 (32 rays per warp, fewer blocks).
-constexpr int kSpreadWarps = 16;
-
-// The share of each warp of a launch over n rays on at most *grid blocks, and
-// the grid that covers them; 0 where the warps take their rays through the
-// queue: the batch exceeds one chunk per resident warp, or the caller chose
-// the chunk.
-unsigned ray_share(const Launch& L, size_t n, int sms, int* grid) {
-  const size_t wpb = (size_t)L.block / 32;
-  if (L.fixed_chunk || n > (size_t)*grid * wpb * 32) return 0;
-  const size_t want = (size_t)sms * kSpreadWarps;
-  const size_t share = std::min<size_t>(32, (n + want - 1) / want);
-  *grid = (int)((n + share * wpb - 1) / (share * wpb));
-  return (unsigned)share;
-}
-
 // The largest batch that wbvh_few takes, in warps of four rays per SM (28,416
 // rays on 148 SMs): at 28,000 rays it took 82 us against 94 in 10,000 random
 // triangles, 47 against 59 on a 131,072-triangle field and 83 against 107 for
