@@ -1138,7 +1138,7 @@ cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
   const size_t o_build = o_pos + up(3 * rec);
   const size_t bytes = o_build + scratch + 256;
   // The map is then written on the stream of this allocation, and its creation
-  // waits for that, so it may be used on any stream.
+  // ends with a wait for that stream, so it may be used on any.
   const cudaError_t e = pool_alloc(&d.slab, bytes, d.device, &d.pooled);
   if (e != cudaSuccess) {
     d.slab = nullptr;
@@ -1276,6 +1276,8 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   }
   if (work_pooled) cudaFreeAsync(work, 0);  // after the build, which used that stream
   else cudaFree(work);
+  // A copy from pageable memory may return while the device still writes.
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) {
     free_photon_map(d);
     delete m;
@@ -1457,6 +1459,7 @@ enc_status enc_photonmap_deserialize(const void* buf, size_t size, int32_t devic
     if (e == cudaSuccess && bytes[i]) e = cudaMemcpy(dst[i], p, bytes[i], cudaMemcpyHostToDevice);
     p += bytes[i];
   }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // as in make_photon_map
   if (e != cudaSuccess) {
     free_photon_map(d);
     delete m;
