@@ -87,6 +87,9 @@ constexpr uint64_t kPoolKeep = 128ull << 20;
 constexpr int kPoolDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kPoolDevices] = {};
+// A small allocation beside the pool.  As long as one lives, another small one and
+// its cudaFree take 2 and 3 us; alone they take 350 and 280.
+void* g_small[kPoolDevices] = {};
 bool g_pool_tried[kPoolDevices] = {};
 
 // The device's pool; null where it has none (then maps use cudaMalloc).
@@ -126,9 +129,24 @@ cudaError_t pool_alloc(void** p, size_t bytes, int device, bool* pooled) {
   return device_malloc(p, bytes);
 }
 
+// Small allocations on the current device `device` are cheap from here on.
+void keep_small(int device) {
+  if (!map_pool(device, true)) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_small[device] && cudaMalloc(&g_small[device], 16) != cudaSuccess) {
+    cudaGetLastError();
+    g_small[device] = nullptr;
+  }
+}
+
 // Gives the device back what its pool keeps.
 void trim_map_pool(int device) {
-  if (cudaMemPool_t pool = map_pool(device, false)) cudaMemPoolTrimTo(pool, 0);
+  cudaMemPool_t pool = map_pool(device, false);
+  if (!pool) return;
+  cudaMemPoolTrimTo(pool, 0);
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  cudaFree(g_small[device]);
+  g_small[device] = nullptr;
 }
 
 template <class T>
@@ -195,7 +213,7 @@ cudaError_t device_malloc(void** p, size_t bytes) {
   if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess &&
       map_pool(device, false)) {
     cudaGetLastError();
-    cudaDeviceSynchronize();  // maps freed in stream order become the pool's to give back
+    cudaStreamSynchronize(0);  // maps freed on that stream become the pool's to give back
     trim_map_pool(device);
     e = cudaMalloc(p, bytes);
   }
@@ -1127,27 +1145,34 @@ namespace {
 // 2,000 / 4,000 photons, 471 / 512 / 544 / 567 us on the device.
 constexpr size_t kHostPhotons = 1024;
 
-// One allocation for a map's arrays, whose sizes photon_layout or a file
-// header has set, and for the device build's scratch; the status word starts
-// at 0.
+// One allocation for a map's arrays, whose sizes photon_layout or a file header
+// has set, and for the device build's scratch; and a small one for its words, of
+// which the status starts at 0.
 cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-  const size_t o_status = up(kGatherSlots * 4), o_box = o_status + 256,
-               o_leaf = o_box + up(4 * d.box_floats), o_pos = o_leaf + up(4 * d.leaf_words),
+  const size_t o_leaf = up(4 * d.box_floats), o_pos = o_leaf + up(4 * d.leaf_words),
                rec = 16 * (size_t)d.n;
   const size_t o_build = o_pos + up(3 * rec);
   const size_t bytes = o_build + scratch + 256;
-  // The map is then written on the stream of this allocation, and its creation
-  // ends with a wait for that stream, so it may be used on any.
-  const cudaError_t e = pool_alloc(&d.slab, bytes, d.device, &d.pooled);
+  keep_small(d.device);
+  cudaError_t e = device_malloc(&d.words, kGatherSlots * 4 + 16);
   if (e != cudaSuccess) {
-    d.slab = nullptr;
+    d.words = nullptr;
     return e;
   }
+  // The map is then written on the stream of this allocation, and its creation
+  // ends with a wait for that stream, so it may be used on any.
+  e = pool_alloc(&d.slab, bytes, d.device, &d.pooled);
+  if (e != cudaSuccess) {
+    d.slab = nullptr;
+    cudaFree(d.words);
+    d.words = nullptr;
+    return e;
+  }
+  d.d_counter = static_cast<uint32_t*>(d.words);
+  d.d_status = d.d_counter + kGatherSlots;
   char* base = static_cast<char*>(d.slab);
-  d.d_counter = reinterpret_cast<uint32_t*>(base);
-  d.d_status = reinterpret_cast<uint32_t*>(base + o_status);
-  d.d_box = reinterpret_cast<float*>(base + o_box);
+  d.d_box = reinterpret_cast<float*>(base);
   d.d_leaf = reinterpret_cast<uint32_t*>(base + o_leaf);
   d.d_pos4 = reinterpret_cast<float*>(base + o_pos);
   d.d_nrm4 = reinterpret_cast<float*>(base + o_pos + rec);
@@ -1156,16 +1181,19 @@ cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
   return cudaMemset(d.d_status, 0, 16);
 }
 
-// A map may still be read on any stream of its device when it is destroyed;
-// cudaFree waits for them by itself.
+// A map may still be read on any stream of its device when it is destroyed.
+// cudaFree of its words waits for them all, and does so while other threads
+// capture graphs, which a cudaDeviceSynchronize would spoil.  Where cudaFree is
+// refused (another thread captures in the mode that forbids it), the memory stays.
 void free_photon_map(DevPhotonMap& d) {
-  if (d.pooled) {
-    cudaDeviceSynchronize();
+  if (cudaFree(d.words) != cudaSuccess) {
+    cudaGetLastError();
+  } else if (d.pooled) {
     cudaFreeAsync(d.slab, 0);
   } else {
     cudaFree(d.slab);
   }
-  d.slab = nullptr;
+  d.words = d.slab = nullptr;
 }
 
 // Whether kernels on `device` can read bytes at p: inside one of its own

@@ -54,6 +54,7 @@ void build_photon_tree(const float* pos, const float* nrm, const float* power, s
 constexpr int kGatherSlots = 256;
 
 struct DevPhotonMap {
+  void* words = nullptr;       // the queue heads and the status word
   void* slab = nullptr;        // the one allocation every array below lies in
   bool pooled = false;         // it came from the device's pool of map memory
   void* build = nullptr;       // ... and the device build's scratch, if it has that
