@@ -414,9 +414,9 @@ enc_status enc_accel_build(enc_scene scene, const enc_build_opts* opts, int32_t 
     set_error(std::string("enc_accel_build: ") + ex.what());
     return ENC_ERR_INVALID_ARG;
   }
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_status, 16);
+  if (e == cudaSuccess) e = device_malloc((void**)&d.d_status, 16);
   if (e == cudaSuccess) e = cudaMemset(d.d_status, 0, 16);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_counter, kQueueSlots * sizeof(uint32_t));
+  if (e == cudaSuccess) e = device_malloc((void**)&d.d_counter, kQueueSlots * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(d.d_counter, 0, kQueueSlots * sizeof(uint32_t));
   if (e != cudaSuccess) {
     free_dev(d);
@@ -705,9 +705,9 @@ enc_status enc_accel_deserialize(const void* buf, size_t size, int32_t device, e
   }
   d.node_bytes = wbvh ? h.node_bytes : h.node_bytes + h.items_bytes;
   d.tri_bytes = h.tri_bytes;
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_status, 16);
+  if (e == cudaSuccess) e = device_malloc((void**)&d.d_status, 16);
   if (e == cudaSuccess) e = cudaMemset(d.d_status, 0, 16);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d.d_counter, kQueueSlots * sizeof(uint32_t));
+  if (e == cudaSuccess) e = device_malloc((void**)&d.d_counter, kQueueSlots * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(d.d_counter, 0, kQueueSlots * sizeof(uint32_t));
   if (e != cudaSuccess) {
     free_dev(d);
@@ -1716,7 +1716,7 @@ enc_status enc_batch_create(const enc_batch_item* items, uint32_t nitems,
   cudaError_t e = upload(&b->d_scenes, scenes.data(), scenes.size());
   if (e == cudaSuccess) e = upload(&b->d_batches, batches.data(), batches.size());
   if (e == cudaSuccess) e = upload(&b->d_starts, starts.data(), starts.size());
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_words, 16);
+  if (e == cudaSuccess) e = device_malloc((void**)&b->d_words, 16);
   if (e == cudaSuccess) e = cudaMemset(b->d_words, 0, 16);
   if (e != cudaSuccess) {
     batch_free(b);
