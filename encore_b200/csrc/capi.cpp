@@ -139,6 +139,12 @@ void keep_small(int device) {
   }
 }
 
+// Work on the memory has ended or was put on the legacy default stream.
+void pool_free(void* p, bool pooled) {
+  if (pooled) cudaFreeAsync(p, 0);
+  else cudaFree(p);
+}
+
 // Gives the device back what its pool keeps.
 void trim_map_pool(int device) {
   cudaMemPool_t pool = map_pool(device, false);
@@ -1146,14 +1152,12 @@ namespace {
 constexpr size_t kHostPhotons = 1024;
 
 // One allocation for a map's arrays, whose sizes photon_layout or a file header
-// has set, and for the device build's scratch; and a small one for its words, of
-// which the status starts at 0.
-cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
+// has set, and a small one for its words, of which the status starts at 0.
+cudaError_t alloc_photon_map(DevPhotonMap& d) {
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   const size_t o_leaf = up(4 * d.box_floats), o_pos = o_leaf + up(4 * d.leaf_words),
                rec = 16 * (size_t)d.n;
-  const size_t o_build = o_pos + up(3 * rec);
-  const size_t bytes = o_build + scratch + 256;
+  const size_t bytes = o_pos + up(3 * rec) + 256;
   keep_small(d.device);
   cudaError_t e = device_malloc(&d.words, kGatherSlots * 4 + 16);
   if (e != cudaSuccess) {
@@ -1177,7 +1181,6 @@ cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
   d.d_pos4 = reinterpret_cast<float*>(base + o_pos);
   d.d_nrm4 = reinterpret_cast<float*>(base + o_pos + rec);
   d.d_pow4 = reinterpret_cast<float*>(base + o_pos + 2 * rec);
-  d.build = scratch ? base + o_build : nullptr;
   return cudaMemset(d.d_status, 0, 16);
 }
 
@@ -1188,10 +1191,8 @@ cudaError_t alloc_photon_map(DevPhotonMap& d, size_t scratch) {
 void free_photon_map(DevPhotonMap& d) {
   if (cudaFree(d.words) != cudaSuccess) {
     cudaGetLastError();
-  } else if (d.pooled) {
-    cudaFreeAsync(d.slab, 0);
   } else {
-    cudaFree(d.slab);
+    pool_free(d.slab, d.pooled);
   }
   d.words = d.slab = nullptr;
 }
@@ -1254,15 +1255,19 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   d.device = device;
   photon_layout(n, &d);
   const size_t bytes = 12 * n;
+  cudaError_t e = alloc_photon_map(d);
+  // The device build's scratch; without room for it the host builds the map.
   bool build = n > kHostPhotons;
-  cudaError_t e = alloc_photon_map(d, build ? photon_build_scratch(n) : 0);
-  if (e == cudaErrorMemoryAllocation && build) {  // the host build needs no scratch
+  void* scratch = nullptr;
+  bool scratch_pooled = false;
+  if (e == cudaSuccess && build &&
+      pool_alloc(&scratch, photon_build_scratch(n), device, &scratch_pooled) != cudaSuccess) {
     cudaGetLastError();
+    scratch = nullptr;
     build = false;
-    e = alloc_photon_map(d, 0);
   }
-  // Photons that a kernel cannot read where they are get copied for the build;
-  // without room for the copy the host builds the map.
+  // Photons that a kernel cannot read where they are get copied for the build,
+  // or the host builds the map.
   bool direct = on_device && build;
   for (int i = 0; i < 3 && direct; ++i) direct = readable_on(src[i], bytes, device);
   void* work = nullptr;
@@ -1283,7 +1288,7 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
     }
     bool refused = false;
     if (e == cudaSuccess)
-      e = (cudaError_t)build_photon_device(in[0], in[1], in[2], d, d.build, &refused);
+      e = (cudaError_t)build_photon_device(in[0], in[1], in[2], d, scratch, &refused);
     if (refused) build = false;
   }
   if (build || e != cudaSuccess) {
@@ -1302,8 +1307,8 @@ enc_status make_photon_map(const float* const src[3], bool on_device, size_t n, 
   } else {
     e = host_photon_map(src[0], src[1], src[2], d, what);
   }
-  if (work_pooled) cudaFreeAsync(work, 0);  // after the build, which used that stream
-  else cudaFree(work);
+  pool_free(work, work_pooled);
+  pool_free(scratch, scratch_pooled);
   // A copy from pageable memory may return while the device still writes.
   if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) {
@@ -1479,7 +1484,7 @@ enc_status enc_photonmap_deserialize(const void* buf, size_t size, int32_t devic
   d.box_floats = h.box_floats;
   d.leaf_words = h.leaf_words;
   const char* p = static_cast<const char*>(buf) + sizeof(h);
-  cudaError_t e = alloc_photon_map(d, 0);
+  cudaError_t e = alloc_photon_map(d);
   void* dst[5] = {d.d_box, d.d_leaf, d.d_pos4, d.d_nrm4, d.d_pow4};
   const size_t bytes[5] = {4 * h.box_floats, 4 * h.leaf_words, 16 * (size_t)h.n,
                            16 * (size_t)h.n, 16 * (size_t)h.n};

@@ -57,7 +57,6 @@ struct DevPhotonMap {
   void* words = nullptr;       // the queue heads and the status word
   void* slab = nullptr;        // the one allocation every array below lies in
   bool pooled = false;         // it came from the device's pool of map memory
-  void* build = nullptr;       // ... and the device build's scratch, if it has that
   float* d_box = nullptr;      // PhotonHost::box
   uint32_t* d_leaf = nullptr;  // PhotonHost::leaf
   int nlevels = 0;
