@@ -21,7 +21,7 @@ struct enc_accel_s {
   enc::WaveScratch wave;  // photon tracer scratch
   enc::WBVHHost host;  // wide BVH kept on the host for refits (its tree; a device refit
                        // leaves the boxes here as they were)
-  enc::RefitScratch refit;
+  enc::RefitPlan refit;
   std::mutex mu;  // serialises the host-buffer forms (shared staging buffers)
   void* d_stage_in = nullptr;
   void* d_stage_out = nullptr;
@@ -76,10 +76,11 @@ enc_status cuda_fail(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(e_, what); \
   } while (0)
 
-// Memory of photon maps.  A renderer makes a map per frame, and a cudaMalloc
-// and a cudaFree take about 0.35 and 0.3 ms (several times that on a busy host),
-// a third of making and using a map of 500,000 photons; so a map's allocation
-// comes from a pool per device that keeps up to kPoolKeep bytes of freed maps.
+// Memory of photon maps and refits.  A renderer makes a map and refits a scene per
+// frame, and a cudaMalloc and a cudaFree take about 0.35 and 0.3 ms (several times
+// that on a busy host), a third of making and using a map of 500,000 photons; so a
+// map's arrays and a build's or refit's scratch come from a pool per device that
+// keeps up to kPoolKeep bytes of what was freed.
 // The kept memory goes back to the device when an accelerator on it is
 // destroyed and when an allocation of this library does not fit.  The pool
 // itself serialises its callers.
@@ -118,17 +119,6 @@ cudaMemPool_t map_pool(int device, bool create) {
   return g_pool[device];
 }
 
-// An allocation from the pool of the current device `device` (cudaMalloc where
-// it has none), on the legacy default stream.
-cudaError_t pool_alloc(void** p, size_t bytes, int device, bool* pooled) {
-  cudaMemPool_t pool = map_pool(device, true);
-  *pooled = pool && cudaMallocFromPoolAsync(p, bytes, pool, 0) == cudaSuccess;
-  if (*pooled) return cudaSuccess;
-  cudaGetLastError();
-  *p = nullptr;
-  return device_malloc(p, bytes);
-}
-
 // Small allocations on the current device `device` are cheap from here on.
 void keep_small(int device) {
   if (!map_pool(device, true)) return;
@@ -139,16 +129,11 @@ void keep_small(int device) {
   }
 }
 
-// Work on the memory has ended or was put on the legacy default stream.
-void pool_free(void* p, bool pooled) {
-  if (pooled) cudaFreeAsync(p, 0);
-  else cudaFree(p);
-}
-
 // Gives the device back what its pool keeps.
 void trim_map_pool(int device) {
   cudaMemPool_t pool = map_pool(device, false);
   if (!pool) return;
+  cudaStreamSynchronize(0);  // the frees on that stream have to be seen done first
   cudaMemPoolTrimTo(pool, 0);
   std::lock_guard<std::mutex> lk(g_pool_mu);
   cudaFree(g_small[device]);
@@ -219,11 +204,24 @@ cudaError_t device_malloc(void** p, size_t bytes) {
   if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess &&
       map_pool(device, false)) {
     cudaGetLastError();
-    cudaStreamSynchronize(0);  // maps freed on that stream become the pool's to give back
     trim_map_pool(device);
     e = cudaMalloc(p, bytes);
   }
   return e;
+}
+
+cudaError_t pool_alloc(void** p, size_t bytes, int device, bool* pooled) {
+  cudaMemPool_t pool = map_pool(device, true);
+  *pooled = pool && cudaMallocFromPoolAsync(p, bytes, pool, 0) == cudaSuccess;
+  if (*pooled) return cudaSuccess;
+  cudaGetLastError();
+  *p = nullptr;
+  return device_malloc(p, bytes);
+}
+
+void pool_free(void* p, bool pooled) {
+  if (pooled) cudaFreeAsync(p, 0);
+  else cudaFree(p);
 }
 
 const DevAccel* accel_device_view(enc_accel a) { return a ? &a->dev : nullptr; }
@@ -738,7 +736,6 @@ enc_status enc_accel_destroy(enc_accel a) {
   DeviceScope ds(a->dev.device);
   free_dev(a->dev);
   free_wave_scratch(&a->wave);
-  free_refit_scratch(&a->refit);
   cudaFree(a->d_stage_in);
   cudaFree(a->d_stage_od);
   cudaFree(a->d_stage_out);

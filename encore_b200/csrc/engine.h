@@ -183,21 +183,17 @@ float box_pad(const float lo[3], const float hi[3], float maxabs);
 // index out of range.
 bool refit_levels_of(const WBVHHost& h, std::vector<uint32_t>& start);
 
-// Device refit (refit.cu): its scratch, kept with the accelerator once it has
-// been refitted, and the tree's levels.
-struct RefitScratch {
-  void* mem = nullptr;
-  size_t bytes = 0;
+// Device refit (refit.cu): the tree's levels, found at the first one.
+struct RefitPlan {
   bool planned = false, usable = false;
   std::vector<uint32_t> level_start;
 };
-void free_refit_scratch(RefitScratch* r);
 // Refits `d` (a wide BVH whose tree is `host`) in place; lo, hi: the scene's
 // new bounds.  *done = false with status 0: nothing was changed, and the host
 // refit has to do it (a table refit_levels_of refuses, a coordinate that is not
 // finite or too large for a grid, no memory for the scratch).  Returns a CUDA
 // error code; `d.device` must be current.
-int refit_device(const DevAccel& d, const WBVHHost& host, RefitScratch* r, const float* tri_verts,
+int refit_device(const DevAccel& d, const WBVHHost& host, RefitPlan* r, const float* tri_verts,
                  float lo[3], float hi[3], bool* done);
 
 // Launch parameters after defaults are applied.
@@ -295,8 +291,13 @@ int launch_multi_any(const MultiLaunch& m, const Launch& L, void* stream);
 int device_sm_count(int device);
 
 // cudaMalloc on the current device; if that does not fit, once more after the
-// memory kept for photon maps has been given back (capi.cpp).
+// memory kept for photon maps and refits has been given back (capi.cpp).
 cudaError_t device_malloc(void** p, size_t bytes);
+// An allocation from the pool of the current device `device` (device_malloc where
+// it has none), on the legacy default stream; and its end, after work on the
+// memory that has ended or was put on that stream.
+cudaError_t pool_alloc(void** p, size_t bytes, int device, bool* pooled);
+void pool_free(void* p, bool pooled);
 
 // Error reporting (capi.cpp).
 void set_error(const std::string& msg);

@@ -246,15 +246,17 @@ cudaError_t run_levels(const Levels& lv, int nlevels, uint8_t* nodes, const floa
   return cudaSuccess;
 }
 
+struct Scratch {
+  void* p = nullptr;
+  bool pooled = false;
+  ~Scratch() {
+    if (p) pool_free(p, pooled);
+  }
+};
+
 }  // namespace
 
-void free_refit_scratch(RefitScratch* r) {
-  cudaFree(r->mem);
-  r->mem = nullptr;
-  r->bytes = 0;
-}
-
-int refit_device(const DevAccel& d, const WBVHHost& host, RefitScratch* r, const float* tri_verts,
+int refit_device(const DevAccel& d, const WBVHHost& host, RefitPlan* r, const float* tri_verts,
                  float lo[3], float hi[3], bool* done) {
   *done = false;
   if (!r->planned) {
@@ -266,16 +268,14 @@ int refit_device(const DevAccel& d, const WBVHHost& host, RefitScratch* r, const
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   const size_t o_box = up(36 * nt), o_node = o_box + up(24 * nt), o_out = o_node + up(24 * nn);
   const size_t need = o_out + 256;
-  if (r->bytes < need) {
-    free_refit_scratch(r);
-    if (device_malloc(&r->mem, need) != cudaSuccess) {
-      cudaGetLastError();  // no room for the scratch: the host refit needs none
-      r->mem = nullptr;
-      return 0;
-    }
-    r->bytes = need;
+  // Taken for this call alone: on the legacy default stream, as all that uses it.
+  Scratch mem;
+  if (pool_alloc(&mem.p, need, d.device, &mem.pooled) != cudaSuccess) {
+    cudaGetLastError();  // no room for the scratch: the host refit needs none
+    mem.p = nullptr;
+    return 0;
   }
-  char* base = static_cast<char*>(r->mem);
+  char* base = static_cast<char*>(mem.p);
   float* verts = reinterpret_cast<float*>(base);
   float2* tri_boxes = reinterpret_cast<float2*>(base + o_box);
   float2* node_boxes = reinterpret_cast<float2*>(base + o_node);
