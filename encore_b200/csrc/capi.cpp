@@ -1143,9 +1143,10 @@ enc_status enc_accel_count_visits(enc_accel a, const float* d_rays, size_t nrays
 
 namespace {
 
-// Up to this many photons a map is built on the host, where the device build's
-// launches take longer: 436 / 497 / 641 / 849 us on the host for 100 / 1,000 /
-// 2,000 / 4,000 photons, 471 / 512 / 544 / 567 us on the device.
+// Up to this many photons a map is built on the host: for 100 / 500 / 1,000 / 2,000 /
+// 4,000 photons in host memory creating it takes 63 / 80 / 128 / 226 / 476 us that
+// way, and 84 / 100 / 124 / 171 / 227 us with the device build.  (Photons in device
+// memory, 93 / 120 / 183 / 281 / 532 against 47 / 60 / 73 / 103 / 120, keep the rule.)
 constexpr size_t kHostPhotons = 1024;
 
 // One allocation for a map's arrays, whose sizes photon_layout or a file header

@@ -20,14 +20,14 @@
 //
 // What bounds it is instruction issue, not memory (L2 holds what it reads).  A
 // bounded max-heap across the warp's registers, whose maximum every accepted
-// photon replaced with two warp reductions, took 911 us for 300,007 queries of
-// k = 50 in a room of 400,000 photons, 1,346 us for 100,007 of k = 256, and 7.6 ms
-// for 1M of k = 50 that find 600 photons each; the buffer takes 577, 621 us and
-// 3.4 ms, and one query at a time per warp where there are few 18 instead of 43
+// photon replaced with two warp reductions, took 916 us for 300,007 queries of
+// k = 50 in a room of 400,000 photons, 1,434 us for 100,007 of k = 256, and 7.6 ms
+// for 1M of k = 50 that find 600 photons each; the buffer takes 620, 765 us and
+// 4.5 ms, and one query at a time per warp where there are few 24 instead of 77
 // us for 1,007.  `full` = k + max(16, 3k/4): more photons per selection against
-// a radius that shrinks later.  k + 0 / 8 / 16 / 32 / 64 for those: 642 / 611 / 599 /
-// 573 / 572, 792 / 731 / 699 / 621 / 621 us, 4.0 / 3.8 / 3.5 / 3.4 / 3.2 ms; for k = 8:
-// 338 / 334 / 325 / 343 / 349 us.
+// a radius that shrinks later.  k + 0 / 8 / 16 / 32 / 64 for those: 713 / 666 / 648 /
+// 621 / 617, 995 / 901 / 835 / 765 / 764 us, 5.6 / 5.1 / 4.7 / 4.5 / 4.4 ms; for k = 8:
+// 373 / 364 / 359 / 368 / 368 us.  Noting the dropped ties (heap_insert) costs 1.4 %.
 //
 // Acceptance is the reference's: FP32 dist^2 = (x*x + y*y) + z*z with separate
 // roundings, dist^2 < r^2, and the stored surface normal equal to the query

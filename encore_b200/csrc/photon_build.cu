@@ -14,8 +14,8 @@
 // pivot and, from the right, at those that are not larger; they exchange the m-th
 // of the one with the m-th of the other while it lies to its left.  So an element's
 // partner follows from the count of the first kind before it and of the second
-// behind it.  What remains (three elements, or the heap) is the library's own
-// code.
+// behind it.  The last three elements are put in order, equal ones left as they
+// are; the heap is the library's own code.
 //
 //   * Ranges of more than kShared photons: one cluster of blocks per range narrows
 //     the selection in device memory, and its first block ends it in shared memory
@@ -29,10 +29,10 @@
 // What bounds it: the length of the chain.  A level takes some eight to fifteen
 // partitions, one after another, of about 2,000 cycles in a block (four barriers,
 // and little between them) and 17,000 to 40,000 in a cluster.  500,000 photons: 45 ms
-// on the host, 0.94 ms here, 0.55 of them in the five levels of split_cluster, 0.17
-// in the four of split_block and 0.07 in split_ranges (clusters of 16 blocks: no
-// faster; rounds of launches over the whole device in their place: 1.42 ms; fewer
-// warps as a block's range shrinks: no faster).  A build that sorts the photons
+// on the host, 0.94 ms here (in a profile 0.62 ms in the five levels of
+// split_cluster, 0.17 in the four of split_block, 0.07 in split_ranges).  Clusters of
+// 16 blocks, and fewer warps as a block's range shrinks, were no faster; rounds of
+// launches over the whole device in place of the clusters took 1.42 ms.  A build that sorts the photons
 // along each axis once and splits the lists took 0.51 ms, but orders equal
 // coordinates and a leaf's photons otherwise, and gathers with photons at equal
 // distances then differed.
@@ -425,18 +425,6 @@ __device__ __forceinline__ Tile tile_of(uint32_t tiles) {
   return Tile{blockIdx.x / tiles, blockIdx.x % tiles};
 }
 
-// A range's selection between two rounds: what is left of it, the partitions left,
-// and the last round's pivot and result.
-struct PartState {
-  uint32_t f, l;
-  int depth;
-  uint32_t active;  // this round partitions it
-  uint32_t at;      // the pivot's place; it goes to f, and the element of f to `at`
-  Elem pivot, front;
-  uint32_t plain;   // the element at `at` is exchanged with no other
-  uint32_t swaps, cut;
-};
-
 __global__ void __launch_bounds__(kThreads) range_extent(const float* __restrict__ pos,
                                                          const Elem* __restrict__ w, uint32_t n,
                                                          int level, uint32_t tiles, uint32_t* ext) {
@@ -675,10 +663,6 @@ __global__ void __launch_bounds__(kThreads) write_boxes(float* box, uint32_t cou
   }
   put_bounds(lo, hi, box, pad, j, lane);
 }
-
-}  // namespace
-
-namespace {
 
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 uint32_t most_in_range(size_t n, int level) {

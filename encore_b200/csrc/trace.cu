@@ -1,7 +1,7 @@
 // Ray traversal kernels for sm_100a.
 //
-//  * wbvh_trace<W, CLAMP, ANY, COUNT, MULTI, LANE>: persistent warps over the
-//    quantised wide BVH.  Each warp takes rays from a global atomic queue in
+//  * wbvh_trace<W, CLAMP, ANY, COUNT, MULTI, LANE, ORD, WAIT>: persistent warps
+//    over the quantised wide BVH.  Each warp takes rays from a global atomic queue in
 //    chunks and hands them to idle lanes as lanes finish (no lane waits for
 //    the slowest ray of a batch).  The traversal stack lives in shared
 //    memory, one column per thread.  A visited node continues with its first
@@ -12,7 +12,10 @@
 //    children by octant (the builder places each child in the slot of its
 //    octant, so slot k ^ octm for k = 0..7 is roughly front to back for a ray
 //    with direction sign bits octm); widths 2 and 4 sort hit children by
-//    entry distance.  MULTI launches trace many scenes' batches at once.
+//    entry distance.  MULTI launches trace many scenes' batches at once; ORD
+//    takes the rays in a given order; WAIT lets lanes at leaves wait for a fuller
+//    triangle round.
+//  * wbvh_few<CLAMP, ANY>: small batches at width 8, eight lanes per ray.
 //  * kd_trace<CLAMP>: the reference's kd-tree walk (Kdtree.cpp:682-784), one
 //    lane per ray with the leaves' items tested by the whole warp, over the
 //    flattened kd layout.  Bit-exact parity mode.
@@ -1539,7 +1542,10 @@ bool few_rays(const Launch& L, size_t n, int sms) {
 // 1,083 without.  Where a visit tests more, rounds are fuller anyway: 1.84M bounce
 // rays on 100,000 random triangles (1.05) took 480 us against 468, 4M on 1M (2.1)
 // 6,210 against 6,049; fields of 20,000 to 2M triangles lie at 0.36 to 0.51 and gain
-// 1.4 to 6 %.  Any hit, at 9 blocks per SM too: 4M / 2M / 1M rays over fields 666 ->
+// 1.4 to 6 %.  The line lies where neither form loses: from 600,000 to 1M rays closest
+// hit gains 0 to 3 % on those trees, but any hit loses 0.7 to 3.5 % on 10,000 random
+// triangles, 1 % at 1M still, and gains 1 to 3 % on the fields from 700,000 on.
+// Any hit, at 9 blocks per SM too: 4M / 2M / 1M rays over fields 666 ->
 // 609 / 305 -> 288 / 164 -> 160 us, 2M on 2,000 / 10,000 / 20,000 random triangles
 // 446 -> 434 / 721 -> 714 / 757 -> 753, 1.5M on 100,000 656 -> 669; 300,000 rays 62 ->
 // 64; where no ray is blocked and most leave the field at once (4.18M toward a light

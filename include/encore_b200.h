@@ -495,6 +495,10 @@ enc_status enc_photonmap_create_device(const float* d_pos, const float* d_nrm, c
 enc_status enc_photonmap_create(const float* pos, const float* normal, const float* power,
                                 size_t nphotons, int32_t caustic, int32_t device,
                                 enc_photonmap* out);
+/* Waits for calls that still read the map.  Up to 128 MiB per device of what
+ * destroyed maps and finished refits used stay with the library for the next
+ * ones; the device gets them back when an accelerator on it is destroyed, or
+ * when an allocation of this library would fail without them. */
 enc_status enc_photonmap_destroy(enc_photonmap map);
 /* A balanced photon map saved as a byte image and loaded without the host
  * balance (enc_accel_serialize's counterpart for photon maps; buf = NULL
