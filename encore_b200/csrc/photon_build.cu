@@ -589,16 +589,21 @@ __global__ void __launch_bounds__(kThreads) split_ranges(const float* __restrict
   for (uint32_t i = threadIdx.x; i < c; i += kThreads) order[all.b + i] = s_id[s_elem[i].id];
 }
 
-// The bounds of a warp's 32 boxes to item j of a level's arrays.
+// The bounds of a warp's 32 boxes to item j of a level's arrays.  Of equal bounds
+// the first lane's is written: a zero's sign is the host build's then.
 __device__ __forceinline__ void put_bounds(float (&lo)[3], float (&hi)[3], float* box, uint32_t pad,
                                            uint32_t j, unsigned lane) {
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1)
+  for (int a = 0; a < 3; ++a) {
+    float least = lo[a], most = hi[a];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      lo[a] = fminf(lo[a], __shfl_xor_sync(kFull, lo[a], d));
-      hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFull, hi[a], d));
+    for (int d = 16; d > 0; d >>= 1) {
+      least = fminf(least, __shfl_xor_sync(kFull, least, d));
+      most = fmaxf(most, __shfl_xor_sync(kFull, most, d));
     }
+    lo[a] = __shfl_sync(kFull, lo[a], __ffs(__ballot_sync(kFull, lo[a] == least)) - 1);
+    hi[a] = __shfl_sync(kFull, hi[a], __ffs(__ballot_sync(kFull, hi[a] == most)) - 1);
+  }
   if (lane < 6) {
     float v = lo[0];
     if (lane == 1) v = lo[1];
