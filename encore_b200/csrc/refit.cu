@@ -246,6 +246,16 @@ cudaError_t run_levels(const Levels& lv, int nlevels, uint8_t* nodes, const floa
   return cudaSuccess;
 }
 
+// A bound of zero has the sign of the axis' first zero, as the host's minima and
+// maxima leave it.  The keys put -0 below +0, so a minimum of +0 or a maximum of -0
+// says that there is no other, and the vertices need not be looked through.
+float zero_bound(const float* v, size_t nverts, int axis, float bound, bool largest) {
+  if (bound != 0.f || std::signbit(bound) == largest) return bound;
+  for (size_t i = 0; i < nverts; ++i)
+    if (v[3 * i + axis] == 0.f) return v[3 * i + axis];
+  return bound;
+}
+
 struct Scratch {
   void* p = nullptr;
   bool pooled = false;
@@ -294,8 +304,8 @@ int refit_device(const DevAccel& d, const WBVHHost& host, RefitPlan* r, const fl
   if (e != cudaSuccess) return (int)e;
   if (k[6]) return 0;  // the host refit says what such coordinates give
   for (int a = 0; a < 3; ++a) {
-    lo[a] = of_key(k[a]);
-    hi[a] = of_key(k[3 + a]);
+    lo[a] = zero_bound(tri_verts, 3 * nt, a, of_key(k[a]), false);
+    hi[a] = zero_bound(tri_verts, 3 * nt, a, of_key(k[3 + a]), true);
   }
   float maxabs = 0.f;
   for (int a = 0; a < 3; ++a) maxabs = std::max(maxabs, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
